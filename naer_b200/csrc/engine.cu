@@ -142,6 +142,12 @@ Engine::~Engine() {
     f(d_ev_part_);
     f(d_ovf_part_);
     f(d_raster_);
+    f(d_gchunks_);
+    f(d_gcnt_);
+    f(d_gbits_);
+    f(d_gq_);
+    f(d_gsegs_);
+    f(d_gtot_);
     for (auto ev : timer_events_) cudaEventDestroy(ev);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (h_pinned_) cudaFreeHost(h_pinned_);
@@ -797,7 +803,8 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
         }
         d.ring_key_base = key_base;
         key_base += (uint64_t)n.ring_slots * n.n_storage;
-        h_nets_.push_back(d);
+        d.pop_first = (uint32_t)pops.size();
+        d.max_row = (uint32_t)std::min<uint64_t>(n.max_row_padded, 0xFFFFFFFFu);
         qcap += n.n_storage;
         id_offsets_.push_back((uint32_t)id_off);
         const auto& P = n.params;
@@ -833,6 +840,13 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
             for (uint32_t f = ps.storage_base; f < ps.storage_base + ps.size; f += kLifChunk)
                 chunks.push_back(ChunkDev{pidx, f, ps.storage_base + ps.size, ni});
         }
+        d.pop_count = (uint32_t)pops.size() - d.pop_first;
+        // no spike reaches a neuron in less than the smallest delay
+        d.window = kGroupMaxWindow;
+        for (const ConnSpec& c : n.conns)
+            if (n.pops[c.src].size && n.pops[c.dst].size) d.window = std::min(d.window, c.spec.delay_min);
+        if (d.stdp_on) d.window = 1;  // a weight update sees the post-synaptic state of its own step
+        h_nets_.push_back(d);
         id_off += n.n_ids;
         if (id_off > 0xFFFFFFFFull) throw Error(NAER_E_OVERFLOW, "more than 2^32 neuron addresses in one engine");
     }
@@ -849,11 +863,22 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
         }
         if (bytes) NAER_CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_));
     };
+    plan_group(pops);  // sets the networks' k_group fields
     upload(reinterpret_cast<void*&>(d_nets_), nets_bytes_, h_nets_.data(), h_nets_.size() * sizeof(NetDev));
     upload(reinterpret_cast<void*&>(d_pops_), pops_bytes_, pops.data(), pops.size() * sizeof(PopDev));
     upload(reinterpret_cast<void*&>(d_chunks_), chunks_bytes_, chunks.data(), chunks.size() * sizeof(ChunkDev));
 
+    if (group_form_ != kGroupNone) {
+        upload(reinterpret_cast<void*&>(d_gchunks_), gchunks_bytes_, h_chunks_.data(), h_chunks_.size() * sizeof(GroupChunk));
+        upload(reinterpret_cast<void*&>(d_gsegs_), gsegs_bytes_, h_segs_.data(), h_segs_.size() * sizeof(GroupSeg));
+    }
+
+    const EngineDev planned = eng_;
     eng_ = EngineDev{};
+    eng_.group_words = planned.group_words;
+    eng_.group_rows = planned.group_rows;
+    eng_.group_own = planned.group_own;
+    eng_.group_cap = planned.group_cap;
     eng_.n_chunks = (uint32_t)chunks.size();
     eng_.n_nets = (uint32_t)nets.size();
 
@@ -916,14 +941,17 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
         events_base_ += sum_parts(d_ev_part_, ev_part_n_);
         overflow_base_ += sum_parts(d_ovf_part_, ev_part_n_);
     }
-    // per-block regions (k_run, deterministic LIF) or one list of every
-    // neuron at most (k_step)
-    const uint64_t qentries = std::max<uint64_t>((uint64_t)lif_grid_ * region_cap, qcap);
+    // per-block regions (k_run) or one list of every neuron at most (k_step,
+    // k_det_step)
+    const uint64_t qentries = list_kernel ? std::max<uint64_t>(qcap, 1) : std::max<uint64_t>((uint64_t)lif_grid_ * region_cap, qcap);
     if (qentries > 0xFFFFFFFFull) throw Error(NAER_E_OVERFLOW, "spike queue larger than 2^32 entries");
+    const uint64_t gentries = group_form_ != kGroupNone ? group_entries_ : 0;
     for (int i = 0; i < 2; ++i) {
-        regrow(reinterpret_cast<void*&>(d_queue_[i]), queue_bytes_[i], qentries * sizeof(SpikeRec));
+        regrow(reinterpret_cast<void*&>(d_queue_[i]), queue_bytes_[i],
+               std::max(qentries, i == 0 ? gentries : 0) * sizeof(SpikeRec));
         regrow(reinterpret_cast<void*&>(d_qid_[i]), qid_bytes_[i], qentries * sizeof(uint32_t));
-        regrow(reinterpret_cast<void*&>(d_qrow_[i]), qrow_bytes_[i], qentries * sizeof(uint4));
+        regrow(reinterpret_cast<void*&>(d_qrow_[i]), qrow_bytes_[i],
+               std::max(qentries, i == 0 ? gentries : 0) * sizeof(uint4));
         regrow(reinterpret_cast<void*&>(d_counts_[i]), counts_bytes_[i], (lif_grid_ + 1) * sizeof(uint32_t));
         NAER_CK(cudaMemsetAsync(d_counts_[i], 0, (lif_grid_ + 1) * sizeof(uint32_t), stream_));
     }
@@ -954,6 +982,22 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     }
     eng_.ev_part = d_ev_part_;
     eng_.ovf_part = d_ovf_part_;
+    if (group_form_ != kGroupNone) {
+        const uint64_t steps = tuning_.launch_steps;
+        regrow(reinterpret_cast<void*&>(d_gcnt_), gcnt_bytes_, group_blocks_ * 4ull);
+        if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * eng_.group_words * group_per_ * 4ull);
+        regrow(reinterpret_cast<void*&>(d_gq_), gq_bytes_, steps * h_segs_.size() * 4ull);
+        NAER_CK(cudaMemsetAsync(d_gq_, 0, steps * h_segs_.size() * 4ull, stream_));
+        regrow(reinterpret_cast<void*&>(d_gtot_), gtot_bytes_, steps * 4ull);
+        NAER_CK(cudaMemsetAsync(d_gtot_, 0, steps * 4ull, stream_));
+        eng_.group_segs = d_gsegs_;
+        eng_.group_seg_n = (uint32_t)h_segs_.size();
+        eng_.group_tot = d_gtot_;
+        eng_.group_chunks = d_gchunks_;
+        eng_.group_cnt = d_gcnt_;
+        eng_.group_bits = d_gbits_;
+        eng_.group_q = d_gq_;
+    }
     eng_.raster = d_raster_;
     eng_.raster_cap = raster_capacity;
     eng_.lif_grid = lif_grid_;
@@ -992,6 +1036,147 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     if (qentries * std::max(eng_.split_first, eng_.split_rest) > 0xFFFFFFFFull)
         throw Error(NAER_E_OVERFLOW, "spike list times warps per spike exceeds 2^32 work items");
     NAER_CK(cudaStreamSynchronize(stream_));  // tables and buffers complete for every stream
+}
+
+// Whether the installed network steps on k_group, its geometry and tables
+// (pops: its populations, in order).  The lines below were measured on B200,
+// µs per grid step, atomic aggregation; "k_step" includes its k_drive.
+//
+//   cluster of 16 blocks, 1 neuron a lane: at most one chunk a warp (two with
+//     windows of one step, up to 8M synapses).  LIF networks of 5k neurons /
+//     out-degree 100: 3.5 (grid 4.2, k_step 9.5); 12k / 100: 4.4 (4.6, 9.5);
+//     12k / 1000: 6.7 (6.0); plastic 12k / 300: 7.3 (8.4, 10.5); Brunel 5k:
+//     1.44 (1.55, 9.2), 10k: 2.2 (1.6, 9.4)
+//   grid, 1 neuron a lane up to two chunks a warp, else 4: 20k / 500: 5.1 (4 a
+//     lane 6.7, k_step 10.5); 100k / 1000: 9.2 (9.3, 12.0); 400k / 500: 13.9
+//     (12.4, 14.5); Brunel 40k: 3.4 (3.9, 10.4)
+//   k_step from 500k neurons (700k / 300: 17.0, grid 17.0; 1M / 1000: 27.0,
+//     27.4) or 250k with plasticity (300k / 300: 14.1, 14.1), unless windows
+//     are longer than one step
+//   block-local delivery (one barrier a step) up to 500k synapses a block: a
+//     block's share of a step's spikes varies, which costs more than the
+//     barrier saves once it is bound by its reductions (50k / 400: 6.6 against
+//     8.4 with the exchange; 200k / 1000: 11.8 against 11.0)
+void Engine::plan_group(const std::vector<PopDev>& pops) {
+    group_form_ = kGroupNone;
+    group_entries_ = 0;
+    if (aggregation_ == NAER_AGG_DETERMINISTIC || !tuning_.group_allowed() || h_nets_.size() != 1) return;
+    NetDev& d = h_nets_[0];
+    const NetHost& n = *nets_[0];
+    if (d.pop_count == 0 || d.pop_count > kGroupPops || (uint32_t)sm_count_ > kGroupMaxBlocks) return;
+    const uint32_t step_warps = kGroupStepThreads / 32;
+    auto chunks_of = [&](uint32_t per) {
+        uint32_t c = 0;
+        for (uint32_t x = 0; x < d.pop_count; ++x) c += (pops[d.pop_first + x].size + 32 * per - 1) / (32 * per);
+        return c;
+    };
+    auto own_of = [&](uint32_t blocks, uint32_t per) {  // neurons of a block, whole rounds of its warps
+        const uint32_t warps = blocks * step_warps;
+        return (chunks_of(per) + warps - 1) / warps * step_warps * 32 * per;
+    };
+    uint32_t c = 16;
+    const uint32_t chunks = chunks_of(1);
+    const bool cluster = chunks <= c * step_warps ||
+                         (d.window == 1 && chunks <= 2 * c * step_warps && n.synapses <= 8000000ull);
+    if (!cluster) c = (uint32_t)sm_count_;
+    group_per_ = cluster || chunks <= 2 * c * step_warps ? 1 : 4;
+    const uint32_t own = own_of(c, group_per_);
+    // the windows' spike records (32 B each) stay below 256 MB
+    const uint64_t most_entries = 8000000;
+    if (!cluster && (uint64_t)c * own * d.window > most_entries)
+        d.window = (uint32_t)std::max<uint64_t>(1, most_entries / ((uint64_t)c * own));
+    if (!cluster && d.window == 1 && n.n_storage > (d.stdp_on ? 250000u : 500000u)) return;
+    const void* kern = group_kernel(!cluster);
+    int optin = 0;
+    NAER_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+    cudaFuncAttributes fa{};
+    NAER_CK(cudaFuncGetAttributes(&fa, kern));
+    const int most = optin - (int)fa.sharedSizeBytes;
+    NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    if (group_smem_bytes(own, group_per_, false) > (size_t)most) return;
+    const bool rows = group_smem_bytes(own, group_per_, true) <= (size_t)most;
+    group_smem_ = group_smem_bytes(own, group_per_, rows);
+    if (cluster) {
+        NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kGroupThreads);
+        cfg.dynamicSmemBytes = group_smem_;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int active = 0;
+        NAER_CK(cudaOccupancyMaxActiveClusters(&active, kern, &cfg));
+        if (active < 1) return;
+    }
+    group_entries_ = (uint64_t)c * own * d.window;
+    if (group_entries_ > 1000000) {  // not where the device is nearly full
+        size_t free_b = 0, total_b = 0;
+        NAER_CK(cudaMemGetInfo(&free_b, &total_b));
+        if (group_entries_ * 32 > free_b / 2) return;
+    }
+    group_form_ = cluster ? kGroupCluster : kGroupGrid;
+    group_blocks_ = c;
+    h_chunks_.clear();
+    h_segs_.clear();
+    const uint32_t chunk = 32 * group_per_;
+    for (uint32_t x = 0; x < d.pop_count; ++x) {
+        const PopDev& p = pops[d.pop_first + x];
+        const uint32_t flags = (p.type == kPOISSON ? 0u : kGcLif) | (p.rate_hz > 0.0 ? kGcDrawn : 0u);
+        for (uint32_t f = 0; f < p.size; f += chunk)
+            h_chunks_.push_back(GroupChunk{p.storage_base + f, x | std::min(chunk, p.size - f) << 8 | flags});
+    }
+    d.g_chunks = (uint32_t)h_chunks_.size();
+    for (uint32_t f = 0; f < d.g_chunks; f += kGroupSeg)
+        h_segs_.push_back(GroupSeg{f, std::min(kGroupSeg, d.g_chunks - f), d.pop_first});
+    d.local = d.window == 1 && !d.stdp_on && n.synapses <= 500000ull * c ? 1u : 0u;
+    eng_.group_words = d.g_chunks;
+    eng_.group_rows = rows ? 1u : 0u;
+    eng_.group_own = own;
+    eng_.group_cap = own * d.window;
+}
+
+const void* Engine::group_kernel(bool grid) const {
+    if (!grid) return (const void*)k_group<false, 1>;
+    return group_per_ == 4 ? (const void*)k_group<true, 4> : (const void*)k_group<true, 1>;
+}
+
+void Engine::launch_group(uint32_t steps, bool from_ctl) {
+    unsigned long long s0 = from_ctl ? kStepFromCtl : host_step_;
+    const bool grid = group_form_ == kGroupGrid;
+    if (grid) NAER_CK(cudaMemsetAsync(&d_ctl_->bar_arrive, 0, 8, stream_));
+    const bool timed = profiling_ && !from_ctl;
+    if (timed) NAER_CK(cudaEventRecord(timer_event(), stream_));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(group_blocks_);
+    cfg.blockDim = dim3(kGroupThreads);
+    cfg.dynamicSmemBytes = group_smem_;
+    cfg.stream = stream_;
+    cudaLaunchAttribute attr[1];
+    if (grid) {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = group_blocks_;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void* args[3] = {&eng_, &s0, &steps};
+    NAER_CK(cudaLaunchKernelExC(&cfg, group_kernel(grid), args));
+    NAER_CK(cudaGetLastError());
+    if (timed) {
+        NAER_CK(cudaEventRecord(timer_event(), stream_));
+        timer_kinds_.push_back(1);
+    }
+    if (!from_ctl) {
+        ++launches_;
+        host_step_ += steps;
+    }
 }
 
 void Engine::set_tuning(const Tuning& t) {
@@ -1226,8 +1411,12 @@ void Engine::run_launches(uint64_t nsteps) {
     // then the persistent kernel simulates the chunk
     while (nsteps > 0) {
         const uint32_t n = (uint32_t)std::min<uint64_t>(nsteps, tuning_.launch_steps);
-        launch_drive(host_step_, n);
-        launch_run(n);
+        if (group_active()) {
+            launch_group(n, false);
+        } else {
+            launch_drive(host_step_, n);
+            launch_run(n);
+        }
         nsteps -= n;
     }
     NAER_CK(cudaGetLastError());
@@ -1252,8 +1441,12 @@ uint64_t Engine::run_graph(uint64_t nsteps, uint32_t graph_launches) {
         cudaError_t err = cudaSuccess;
         try {
             for (uint32_t i = 0; i < graph_launches; ++i) {
-                launch_drive(kStepFromCtl, L);
-                launch_run_ex(L, true);
+                if (group_active()) {
+                    launch_group(L, true);
+                } else {
+                    launch_drive(kStepFromCtl, L);
+                    launch_run_ex(L, true);
+                }
             }
         } catch (...) {
             cudaGraph_t gdrop = nullptr;
@@ -1272,7 +1465,7 @@ uint64_t Engine::run_graph(uint64_t nsteps, uint32_t graph_launches) {
     while (graph_exec_ && nsteps - done >= per) {
         NAER_CK(cudaGraphLaunch(graph_exec_, stream_));
         host_step_ += per;
-        launches_ += 2ull * graph_launches;
+        launches_ += (group_active() ? 1ull : 2ull) * graph_launches;
         done += per;
     }
     run(nsteps - done);
@@ -1411,6 +1604,8 @@ void Engine::set_barrier_limit(uint64_t limit_ns) {
 
 void Engine::set_barrier_skew(uint64_t skew) {
     DeviceGuard g(device_);
+    drop_graph();
+    bar_skew_ = skew;  // clusters have no barrier that could wait in vain: the grid kernels take over
     const unsigned long long v = skew;
     std::memcpy(h_pinned_ + 66, &v, 8);
     NAER_CK(cudaMemcpyAsync(&d_ctl_->bar_skew, h_pinned_ + 66, 8, cudaMemcpyHostToDevice, stream_));

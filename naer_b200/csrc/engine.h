@@ -120,6 +120,12 @@ struct Tuning {
     uint32_t neuron_state = 0;             // NAER_STATE_AUTO / _SHARED / _GLOBAL: where the step kernel keeps V
     uint32_t step_kernel = 0;              // NAER_KERNEL_SPLIT (k_step) / NAER_KERNEL_TWO_BARRIER (k_run)
     uint32_t bins = 0;                     // k_step shared-memory binning table entries (0 = off)
+
+    // the choices that name a kernel or a geometry of its own are all open
+    bool group_allowed() const {
+        return blocks_per_sm == 0 && scatter_split == 0 && scatter_piece == 0 && neuron_state == 0 && bins == 0 &&
+               step_kernel == 0;
+    }
 };
 
 struct TuneResult {
@@ -222,6 +228,10 @@ public:
 private:
     void build_arrays(NetHost& n);
     std::vector<std::pair<void*, size_t>>* alloc_log_ = nullptr;  // allocations of a build in progress
+    void plan_group(const std::vector<PopDev>& pops);
+    const void* group_kernel(bool grid) const;
+    bool group_active() const { return group_form_ == kGroupGrid || (group_form_ == kGroupCluster && bar_skew_ == 0); }
+    void launch_group(uint32_t steps, bool from_ctl);
     void launch_run(uint32_t steps);
     void launch_drive(uint64_t s_first, uint32_t nsteps);
     void run_launches(uint64_t nsteps);
@@ -285,6 +295,24 @@ private:
     bool profiling_ = false;
     bool use_smem_state_ = false;
     bool split_kernel_ = true;  // k_step (else k_run)
+    // k_group: which form the installed networks step on, its geometry and tables
+    static constexpr uint32_t kGroupNone = 0, kGroupCluster = 1, kGroupGrid = 2;
+    uint32_t group_form_ = kGroupNone;
+    uint32_t group_per_ = 1;       // neurons a lane
+    uint32_t group_blocks_ = 0;    // blocks of the launch
+    size_t group_smem_ = 0;
+    uint64_t group_entries_ = 0;   // spike records of all blocks
+    uint64_t bar_skew_ = 0;
+    std::vector<GroupChunk> h_chunks_;
+    std::vector<GroupSeg> h_segs_;
+    GroupSeg* d_gsegs_ = nullptr;
+    uint32_t* d_gtot_ = nullptr;
+    size_t gsegs_bytes_ = 0, gtot_bytes_ = 0;
+    GroupChunk* d_gchunks_ = nullptr;
+    uint32_t* d_gcnt_ = nullptr;
+    uint32_t* d_gbits_ = nullptr;
+    uint32_t* d_gq_ = nullptr;
+    size_t gchunks_bytes_ = 0, gcnt_bytes_ = 0, gbits_bytes_ = 0, gq_bytes_ = 0;
     // CUDA-event timing of launches while profiling (pairs in launch order)
     std::vector<cudaEvent_t> timer_events_;
     std::vector<int> timer_kinds_;  // 0 drive, 1 step kernel

@@ -41,6 +41,15 @@ constexpr uint32_t kPostWordsMax = 20;
 // (launches recorded once in a CUDA graph and replayed).
 constexpr unsigned long long kStepFromCtl = ~0ull;
 constexpr uint32_t kLifBatch = 4;     // owned chunks whose loads are issued together
+// k_group (group_kernel.cuh)
+constexpr uint32_t kGroupThreads = 512;
+constexpr uint32_t kGroupStepThreads = 384;  // of them, threads that step neurons
+constexpr uint32_t kGroupMaxWindow = 16;  // steps of a window, at most
+constexpr uint32_t kGroupMaxBlocks = 160; // blocks of a group, at most
+constexpr uint32_t kGroupPops = 8;        // populations of a network, at most
+constexpr uint32_t kGroupList = 1024;     // spikes of a window a block keeps in shared memory
+constexpr uint32_t kGroupSeg = 64;        // chunks of a raster segment
+constexpr uint32_t kGcLif = 1u << 16, kGcDrawn = 1u << 17;  // GroupChunk::info: LIF neurons; Poisson counts are drawn
 
 struct PopDev {
     uint32_t net;           // owning net slot
@@ -61,6 +70,20 @@ struct PopDev {
     uint32_t rng_idx_base;  // idx of the first neuron in the generator's index space
     uint32_t z_hi;          // z in [z_hi, 0xFFFFFFFE] => first interval >= window
     uint32_t t0_limit;      // fast path valid while t0 <= t0_limit (no u32 wrap)
+};
+
+// Consecutive neurons of one population, one or four for each lane of a warp
+// (fewer at its end): the piece of a network one warp of k_group steps.
+struct GroupChunk {
+    uint32_t first;  // first storage index
+    uint32_t info;   // index among the network's populations | neurons (1..128) << 8 | kGcLif, kGcDrawn
+};
+
+// Up to kGroupSeg consecutive chunks: the piece of the raster one warp writes.
+struct GroupSeg {
+    uint32_t first;      // first chunk
+    uint32_t count;
+    uint32_t pop_first;  // the network's first population
 };
 
 struct NetDev {
@@ -110,6 +133,13 @@ struct NetDev {
     // (fx_scale = 2^S, fx_inv = 2^-S); both 0 when the ring holds floats
     float fx_scale;
     float fx_inv;
+    // k_group
+    uint32_t window;        // steps per window: the smallest delay (1 with plasticity on), <= kGroupMaxWindow
+    uint32_t pop_first;     // the network's populations: EngineDev::pops [pop_first, pop_first + pop_count)
+    uint32_t pop_count;
+    uint32_t g_chunks;      // entries of EngineDev::group_chunks
+    uint32_t max_row;       // longest padded row
+    uint32_t local;         // 1: a block delivers the spikes of its own neurons (window 1, no plasticity)
     uint32_t pad_;
 };
 
@@ -201,6 +231,19 @@ struct EngineDev {
     uint32_t split_rest;
     uint32_t queue_cap;             // entries of queue[i] / qid[i]
     uint32_t bins;                  // k_step: shared-memory binning table entries (power of 2), 0 = off
+    // k_group
+    const GroupChunk* group_chunks; // the network's chunks, in storage order
+    uint32_t* group_cnt;            // grid form: spikes of each block in the window
+    uint32_t* group_bits;           // [steps][group_words][neurons a lane] spikes of the launch: word k of a chunk =
+                                    // neuron k of each lane
+    const GroupSeg* group_segs;     // its raster segments, in address order
+    uint32_t* group_q;              // [steps][group_seg_n] spikes per step and segment (0 between launches)
+    uint32_t* group_tot;            // [steps] spikes per step (0 between launches)
+    uint32_t group_seg_n;
+    uint32_t group_words;           // its chunks
+    uint32_t group_rows;            // 1: the blocks keep their neurons' row bounds in shared memory
+    uint32_t group_own;             // neurons of a block, at most (a multiple of 32)
+    uint32_t group_cap;             // spike records of a block in one window, at most
 };
 
 }  // namespace naer

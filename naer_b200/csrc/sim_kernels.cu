@@ -1893,3 +1893,5 @@ size_t run_smem_bytes(uint32_t grid, uint32_t own_max, bool smem_state) {
 }
 
 }  // namespace naer
+
+#include "group_kernel.cuh"
