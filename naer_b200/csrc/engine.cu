@@ -2,7 +2,9 @@
 #include <cub/cub.cuh>
 
 #include <atomic>
+#include <functional>
 #include <mutex>
+#include <queue>
 
 #include <algorithm>
 #include <cmath>
@@ -147,6 +149,11 @@ Engine::~Engine() {
     f(d_gbits_);
     f(d_gq_);
     f(d_gsegs_);
+    f(d_gorder_);
+    for (auto st : class_stream_)
+        if (st) cudaStreamDestroy(st);
+    for (auto ev : class_event_)
+        if (ev) cudaEventDestroy(ev);
     f(d_gtot_);
     for (auto ev : timer_events_) cudaEventDestroy(ev);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
@@ -870,15 +877,14 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
 
     if (group_form_ != kGroupNone) {
         upload(reinterpret_cast<void*&>(d_gchunks_), gchunks_bytes_, h_chunks_.data(), h_chunks_.size() * sizeof(GroupChunk));
+        if (h_nets_.size() > 1)
+            upload(reinterpret_cast<void*&>(d_gorder_), gorder_bytes_, h_order_.data(), h_order_.size() * 4ull);
         upload(reinterpret_cast<void*&>(d_gsegs_), gsegs_bytes_, h_segs_.data(), h_segs_.size() * sizeof(GroupSeg));
     }
 
     const EngineDev planned = eng_;
     eng_ = EngineDev{};
     eng_.group_words = planned.group_words;
-    eng_.group_rows = planned.group_rows;
-    eng_.group_own = planned.group_own;
-    eng_.group_cap = planned.group_cap;
     eng_.n_chunks = (uint32_t)chunks.size();
     eng_.n_nets = (uint32_t)nets.size();
 
@@ -955,11 +961,12 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
         regrow(reinterpret_cast<void*&>(d_counts_[i]), counts_bytes_[i], (lif_grid_ + 1) * sizeof(uint32_t));
         NAER_CK(cudaMemsetAsync(d_counts_[i], 0, (lif_grid_ + 1) * sizeof(uint32_t), stream_));
     }
-    regrow(reinterpret_cast<void*&>(d_ev_part_), ev_part_bytes_, scatter_grid_ * sizeof(unsigned long long));
-    regrow(reinterpret_cast<void*&>(d_ovf_part_), ovf_part_bytes_, scatter_grid_ * sizeof(unsigned long long));
-    NAER_CK(cudaMemsetAsync(d_ev_part_, 0, scatter_grid_ * sizeof(unsigned long long), stream_));
-    NAER_CK(cudaMemsetAsync(d_ovf_part_, 0, scatter_grid_ * sizeof(unsigned long long), stream_));
-    ev_part_n_ = scatter_grid_;
+    const uint32_t parts = group_form_ != kGroupNone ? std::max(scatter_grid_, group_blocks_) : scatter_grid_;
+    regrow(reinterpret_cast<void*&>(d_ev_part_), ev_part_bytes_, parts * sizeof(unsigned long long));
+    regrow(reinterpret_cast<void*&>(d_ovf_part_), ovf_part_bytes_, parts * sizeof(unsigned long long));
+    NAER_CK(cudaMemsetAsync(d_ev_part_, 0, parts * sizeof(unsigned long long), stream_));
+    NAER_CK(cudaMemsetAsync(d_ovf_part_, 0, parts * sizeof(unsigned long long), stream_));
+    ev_part_n_ = parts;
     queue_cap_ = (uint32_t)qentries;
     const size_t rbytes = std::max<uint64_t>(raster_capacity, 1) * sizeof(uint2);
     if (rbytes != raster_bytes_) {
@@ -985,7 +992,8 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     if (group_form_ != kGroupNone) {
         const uint64_t steps = tuning_.launch_steps;
         regrow(reinterpret_cast<void*&>(d_gcnt_), gcnt_bytes_, group_blocks_ * 4ull);
-        if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * eng_.group_words * group_per_ * 4ull);
+        NAER_CK(cudaMemsetAsync(&d_ctl_->raster_done, 0, 4, stream_));
+        if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * eng_.group_words * 4ull);
         regrow(reinterpret_cast<void*&>(d_gq_), gq_bytes_, steps * h_segs_.size() * 4ull);
         NAER_CK(cudaMemsetAsync(d_gq_, 0, steps * h_segs_.size() * 4ull, stream_));
         regrow(reinterpret_cast<void*&>(d_gtot_), gtot_bytes_, steps * 4ull);
@@ -1038,8 +1046,50 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     NAER_CK(cudaStreamSynchronize(stream_));  // tables and buffers complete for every stream
 }
 
-// Whether the installed network steps on k_group, its geometry and tables
-// (pops: its populations, in order).  The lines below were measured on B200,
+// 32 x per neurons of one population a warp takes at a time.
+static uint32_t group_chunks(const NetDev& d, const std::vector<PopDev>& pops, uint32_t per) {
+    uint32_t c = 0;
+    for (uint32_t x = 0; x < d.pop_count; ++x) c += (pops[d.pop_first + x].size + 32 * per - 1) / (32 * per);
+    return c;
+}
+// Neurons of one of `blocks` blocks: whole rounds of its stepping warps.
+static uint32_t group_own(const NetDev& d, const std::vector<PopDev>& pops, uint32_t blocks, uint32_t per) {
+    const uint32_t step_warps = kGroupStepThreads / 32, warps = blocks * step_warps;
+    return (group_chunks(d, pops, per) + warps - 1) / warps * step_warps * 32 * per;
+}
+
+// Shared memory of a class; false if its blocks or clusters cannot be
+// resident.
+bool Engine::fit_class(GroupClass& c) {
+    const void* kern = group_kernel(c);
+    int optin = 0;
+    NAER_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+    cudaFuncAttributes fa{};
+    NAER_CK(cudaFuncGetAttributes(&fa, kern));
+    const int most = optin - (int)fa.sharedSizeBytes;
+    NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    if (group_smem_bytes(c.own, c.per, false) > (size_t)most) return false;
+    c.rows = group_smem_bytes(c.own, c.per, true) <= (size_t)most;
+    c.smem = group_smem_bytes(c.own, c.per, c.rows);
+    if (group_form_ == kGroupGrid) return true;
+    NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c.size);
+    cfg.blockDim = dim3(kGroupThreads);
+    cfg.dynamicSmemBytes = c.smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c.size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int active = 0;
+    NAER_CK(cudaOccupancyMaxActiveClusters(&active, kern, &cfg));
+    return active >= 1;
+}
+
+// Geometry of k_group for one network, or false: k_step.  The lines below
+// were measured on B200,
 // µs per grid step, atomic aggregation; "k_step" includes its k_drive.
 //
 //   cluster of 16 blocks, 1 neuron a lane: at most one chunk a warp (two with
@@ -1057,91 +1107,226 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
 //     block's share of a step's spikes varies, which costs more than the
 //     barrier saves once it is bound by its reductions (50k / 400: 6.6 against
 //     8.4 with the exchange; 200k / 1000: 11.8 against 11.0)
-void Engine::plan_group(const std::vector<PopDev>& pops) {
-    group_form_ = kGroupNone;
-    group_entries_ = 0;
-    if (aggregation_ == NAER_AGG_DETERMINISTIC || !tuning_.group_allowed() || h_nets_.size() != 1) return;
+bool Engine::plan_one(const std::vector<PopDev>& pops) {
     NetDev& d = h_nets_[0];
     const NetHost& n = *nets_[0];
-    if (d.pop_count == 0 || d.pop_count > kGroupPops || (uint32_t)sm_count_ > kGroupMaxBlocks) return;
-    const uint32_t step_warps = kGroupStepThreads / 32;
-    auto chunks_of = [&](uint32_t per) {
-        uint32_t c = 0;
-        for (uint32_t x = 0; x < d.pop_count; ++x) c += (pops[d.pop_first + x].size + 32 * per - 1) / (32 * per);
-        return c;
-    };
-    auto own_of = [&](uint32_t blocks, uint32_t per) {  // neurons of a block, whole rounds of its warps
-        const uint32_t warps = blocks * step_warps;
-        return (chunks_of(per) + warps - 1) / warps * step_warps * 32 * per;
-    };
+    const uint32_t step_warps = kGroupStepThreads / 32, chunks = group_chunks(d, pops, 1);
     uint32_t c = 16;
-    const uint32_t chunks = chunks_of(1);
     const bool cluster = chunks <= c * step_warps ||
                          (d.window == 1 && chunks <= 2 * c * step_warps && n.synapses <= 8000000ull);
     if (!cluster) c = (uint32_t)sm_count_;
-    group_per_ = cluster || chunks <= 2 * c * step_warps ? 1 : 4;
-    const uint32_t own = own_of(c, group_per_);
+    if (c > kGroupMaxBlocks) return false;
+    group_form_ = cluster ? kGroupCluster : kGroupGrid;
+    GroupClass k;
+    k.size = c;
+    k.nets = 1;
+    k.per = cluster || chunks <= 2 * c * step_warps ? 1 : 4;
+    k.own = group_own(d, pops, c, k.per);
+    k.stdp = d.stdp_on != 0;
     // the windows' spike records (32 B each) stay below 256 MB
     const uint64_t most_entries = 8000000;
-    if (!cluster && (uint64_t)c * own * d.window > most_entries)
-        d.window = (uint32_t)std::max<uint64_t>(1, most_entries / ((uint64_t)c * own));
-    if (!cluster && d.window == 1 && n.n_storage > (d.stdp_on ? 250000u : 500000u)) return;
-    const void* kern = group_kernel(!cluster);
-    int optin = 0;
-    NAER_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-    cudaFuncAttributes fa{};
-    NAER_CK(cudaFuncGetAttributes(&fa, kern));
-    const int most = optin - (int)fa.sharedSizeBytes;
-    NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    if (group_smem_bytes(own, group_per_, false) > (size_t)most) return;
-    const bool rows = group_smem_bytes(own, group_per_, true) <= (size_t)most;
-    group_smem_ = group_smem_bytes(own, group_per_, rows);
-    if (cluster) {
-        NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(c);
-        cfg.blockDim = dim3(kGroupThreads);
-        cfg.dynamicSmemBytes = group_smem_;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = c;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int active = 0;
-        NAER_CK(cudaOccupancyMaxActiveClusters(&active, kern, &cfg));
-        if (active < 1) return;
-    }
-    group_entries_ = (uint64_t)c * own * d.window;
-    if (group_entries_ > 1000000) {  // not where the device is nearly full
-        size_t free_b = 0, total_b = 0;
-        NAER_CK(cudaMemGetInfo(&free_b, &total_b));
-        if (group_entries_ * 32 > free_b / 2) return;
-    }
-    group_form_ = cluster ? kGroupCluster : kGroupGrid;
-    group_blocks_ = c;
-    h_chunks_.clear();
-    h_segs_.clear();
-    const uint32_t chunk = 32 * group_per_;
-    for (uint32_t x = 0; x < d.pop_count; ++x) {
-        const PopDev& p = pops[d.pop_first + x];
-        const uint32_t flags = (p.type == kPOISSON ? 0u : kGcLif) | (p.rate_hz > 0.0 ? kGcDrawn : 0u);
-        for (uint32_t f = 0; f < p.size; f += chunk)
-            h_chunks_.push_back(GroupChunk{p.storage_base + f, x | std::min(chunk, p.size - f) << 8 | flags});
-    }
-    d.g_chunks = (uint32_t)h_chunks_.size();
-    for (uint32_t f = 0; f < d.g_chunks; f += kGroupSeg)
-        h_segs_.push_back(GroupSeg{f, std::min(kGroupSeg, d.g_chunks - f), d.pop_first});
-    d.local = d.window == 1 && !d.stdp_on && n.synapses <= 500000ull * c ? 1u : 0u;
-    eng_.group_words = d.g_chunks;
-    eng_.group_rows = rows ? 1u : 0u;
-    eng_.group_own = own;
-    eng_.group_cap = own * d.window;
+    if (!cluster && (uint64_t)c * k.own * d.window > most_entries)
+        d.window = (uint32_t)std::max<uint64_t>(1, most_entries / ((uint64_t)c * k.own));
+    if (!cluster && d.window == 1 && n.n_storage > (d.stdp_on ? 250000u : 500000u)) return false;
+    if (!fit_class(k)) return false;
+    group_classes_.assign(1, k);
+    h_order_.assign(1, 0u);
+    return true;
 }
 
-const void* Engine::group_kernel(bool grid) const {
-    if (!grid) return (const void*)k_group<false, 1>;
-    return group_per_ == 4 ? (const void*)k_group<true, 4> : (const void*)k_group<true, 1>;
+// Clusters for several networks: every network gets the smallest cluster with
+// which its step takes at most T, for the T that minimises a launch's length.  The step times are a model
+// fitted to measurements (us, networks of 2k to 45k neurons on 1 to 16
+// blocks): the LIF's rounds of the warps, a chain of 1.3 (static) or 2.7
+// (plastic), and the events at the rates a block delivers them (800 and 260)
+// or the draws (880), whichever is longer.  False if the grid kernel, which
+// steps all networks together, is expected to be faster.
+bool Engine::plan_several(const std::vector<PopDev>& pops) {
+    static const uint32_t sizes[] = {1, 2, 4, 8};  // clusters of 16 crowd the others out (20 of 5k: 8.3, without 7.0)
+    constexpr int kSizes = 4;
+    group_form_ = kGroupCluster;
+    const uint32_t step_warps = kGroupStepThreads / 32;
+    const size_t count = h_nets_.size();
+    auto per_of = [&](const NetDev& d, uint32_t c) { return group_chunks(d, pops, 1) <= 2 * c * step_warps ? 1u : 4u; };
+    int optin = 0;
+    NAER_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+    const size_t smem_most = (size_t)optin - 4096;  // less what the kernel declares itself
+    std::vector<double> t(count * kSizes);
+    double plastic = 0, fixed = 0, neurons = 0;  // events per step, neurons
+    for (size_t i = 0; i < count; ++i) {
+        const NetDev& d = h_nets_[i];
+        double spikes = 0, n = 0, drawn = 0;  // expected spikes per second
+        for (uint32_t x = 0; x < d.pop_count; ++x) {
+            const PopDev& p = pops[d.pop_first + x];
+            n += p.size;
+            drawn += p.rate_hz > 0.0 ? p.size : 0.0;
+            spikes += p.size * (p.type == kPOISSON ? p.rate_hz : p.rate_hz > 0.0 ? 1.0 + std::min(0.6 * p.rate_hz, 50.0) : 8.0);
+        }
+        const double ev = 1e-6 * d.dt_us * (double)nets_[i]->synapses * (spikes / n);
+        (d.stdp_on ? plastic : fixed) += ev;
+        neurons += n;
+        for (int k = 0; k < kSizes; ++k) {
+            const uint32_t c = sizes[k], per = per_of(d, c);
+            const double rounds = (double)group_own(d, pops, c, per) / (32.0 * per * step_warps);
+            const double lif = per == 1 ? 0.55 + 0.37 * rounds : 0.75 + 0.73 * rounds;
+            const double draw = drawn / c / 880.0;
+            const double rest = d.stdp_on ? 2.7 + std::max(1.8 + ev / (c * 260.0), draw)
+                                          : 1.3 + std::max(0.8 + ev / (c * 800.0), draw);
+            // neurons that do not fit one block's shared memory
+            const bool fits = group_smem_bytes(group_own(d, pops, c, per), per, false) <= smem_most;
+            t[i * kSizes + k] = fits ? lif + rest : 1e9;
+        }
+    }
+    // a launch as the device runs it: the clusters, largest first, each on
+    // free SMs for all its steps (clusters of mixed sizes leave some SMs of a
+    // GPC unused: with all 148 planned full, a cluster that finds no place
+    // waits for a whole launch: 40 networks of 30k 17.5 us, with 0.82 14.1)
+    const uint32_t sms = (uint32_t)(0.82 * sm_count_);
+    auto span_of = [&](const std::vector<int>& pick) {
+        std::vector<uint32_t> order(count);
+        for (uint32_t i = 0; i < count; ++i) order[i] = i;
+        std::sort(order.begin(), order.end(), [&](uint32_t l, uint32_t r) {
+            return pick[l] != pick[r] ? pick[l] > pick[r] : t[l * kSizes + pick[l]] > t[r * kSizes + pick[r]];
+        });
+        std::priority_queue<std::pair<double, uint32_t>, std::vector<std::pair<double, uint32_t>>, std::greater<>> busy;
+        uint32_t free = sms;
+        double now = 0, end = 0;
+        for (uint32_t i : order) {
+            const uint32_t c = sizes[pick[i]];
+            while (free < c) {
+                now = busy.top().first;
+                free += busy.top().second;
+                busy.pop();
+            }
+            free -= c;
+            busy.push({now + t[i * kSizes + pick[i]], c});
+            end = std::max(end, now + t[i * kSizes + pick[i]]);
+        }
+        return end;
+    };
+    std::vector<double> targets(t);
+    std::sort(targets.begin(), targets.end());
+    double best = 1e30;
+    std::vector<int> pick(count), best_pick;
+    for (size_t x = 0; x < targets.size(); x += std::max<size_t>(1, targets.size() / 64)) {
+        for (size_t i = 0; i < count; ++i) {
+            int k = 0;
+            while (k + 1 < kSizes && t[i * kSizes + k] > targets[x]) ++k;
+            pick[i] = k;
+        }
+        const double span = span_of(pick);
+        if (span < best && span < 1e8) {
+            best = span;
+            best_pick = pick;
+        }
+    }
+    const double grid = 8.0 + neurons / 3e5 + plastic / 8300.0 + fixed / 28000.0;
+    // measured, clusters / grid (model): 48 networks of up to 50k neurons 29.6 /
+    // 40.4 (21.7 / 39.5), 20 of 5k 7.0 / 10.8 (6.5 / 8.7), 100 of 20k 22.8 /
+    // 26.1 (18.0 / 25.2), 25 of 12k 11.8 / 12.2 (7.1 / 9.7), 10 of 30k 16.7 /
+    // 15.0 (14.0 / 13.3), 5 of 50k 20.5 / 13.0 (21.8 / 12.8)
+    if (best_pick.empty() || best > 0.95 * grid) return false;
+    // classes by cluster size and neurons a lane, the largest clusters first
+    group_classes_.clear();
+    h_order_.clear();
+    for (int k = kSizes - 1; k >= 0; --k)
+        for (uint32_t per : {4u, 1u}) {
+            GroupClass c;
+            c.size = sizes[k];
+            c.per = per;
+            const size_t first = h_order_.size();
+            for (uint32_t i = 0; i < count; ++i) {
+                if (best_pick[i] != k || per_of(h_nets_[i], sizes[k]) != per) continue;
+                h_order_.push_back(i);
+                ++c.nets;
+                c.own = std::max(c.own, group_own(h_nets_[i], pops, sizes[k], per));
+                c.stdp = c.stdp || h_nets_[i].stdp_on;
+            }
+            if (!c.nets) continue;
+            std::stable_sort(h_order_.begin() + first, h_order_.end(),
+                             [&](uint32_t l, uint32_t r) { return nets_[l]->synapses > nets_[r]->synapses; });
+            if (!fit_class(c)) return false;
+            group_classes_.push_back(c);
+        }
+    return true;
+}
+
+// Whether the installed networks step on k_group, and their tables (pops:
+// every network's populations, in order).
+void Engine::plan_group(const std::vector<PopDev>& pops) {
+    group_form_ = kGroupNone;
+    group_entries_ = 0;
+    if (aggregation_ == NAER_AGG_DETERMINISTIC || !tuning_.group_allowed() || h_nets_.empty()) return;
+    bool ok = true;
+    for (const NetDev& d : h_nets_) ok = ok && d.pop_count > 0 && d.pop_count <= kGroupPops;
+    ok = ok && (h_nets_.size() == 1 ? plan_one(pops) : plan_several(pops));
+    // per network: chunks, raster segments, spike records; classes in order
+    h_chunks_.clear();
+    h_segs_.clear();
+    group_blocks_ = 0;
+    uint32_t words = 0;
+    if (ok) {
+        std::vector<const GroupClass*> of(h_nets_.size());
+        size_t at = 0;
+        for (const GroupClass& c : group_classes_) {
+            group_blocks_ += c.nets * c.size;
+            for (uint32_t x = 0; x < c.nets; ++x) of[h_order_[at++]] = &c;
+        }
+        for (size_t i = 0; i < h_nets_.size(); ++i) {  // in address order
+            NetDev& d = h_nets_[i];
+            const GroupClass& c = *of[i];
+            const uint32_t chunk = 32 * c.per;
+            d.g_first = (uint32_t)h_chunks_.size();
+            d.seg_first = (uint32_t)h_segs_.size();
+            words = (words + 3u) & ~3u;
+            d.g_word = words;
+            for (uint32_t x = 0; x < d.pop_count; ++x) {
+                const PopDev& p = pops[d.pop_first + x];
+                const uint32_t flags = (p.type == kPOISSON ? 0u : kGcLif) | (p.rate_hz > 0.0 ? kGcDrawn : 0u);
+                for (uint32_t f = 0; f < p.size; f += chunk)
+                    h_chunks_.push_back(GroupChunk{p.storage_base + f, x | std::min(chunk, p.size - f) << 8 | flags});
+            }
+            d.g_chunks = (uint32_t)h_chunks_.size() - d.g_first;
+            // one network in a cluster: one segment (a warp a step, no counts of segments)
+            const uint32_t seg = h_nets_.size() == 1 && group_form_ == kGroupCluster ? std::max(1u, d.g_chunks) : kGroupSeg;
+            for (uint32_t f = 0; f < d.g_chunks; f += seg)
+                h_segs_.push_back(GroupSeg{d.g_first + f, std::min(seg, d.g_chunks - f), words + f * c.per, c.per, d.pop_first});
+            d.seg_n = (uint32_t)h_segs_.size() - d.seg_first;
+            words += d.g_chunks * c.per;
+            d.local = d.window == 1 && !d.stdp_on && nets_[i]->synapses <= 500000ull * c.size ? 1u : 0u;
+            d.q_cap = group_own(d, pops, c.size, c.per) * d.window;
+            d.q_off = group_entries_;
+            group_entries_ += (uint64_t)d.q_cap * c.size;
+        }
+        eng_.group_words = (words + 3u) & ~3u;
+    }
+    if (ok && group_entries_ > 1000000) {  // not where the device is nearly full
+        size_t free_b = 0, total_b = 0;
+        NAER_CK(cudaMemGetInfo(&free_b, &total_b));
+        ok = group_entries_ * 32 <= free_b / 2;
+    }
+    if (!ok) {
+        group_form_ = kGroupNone;
+        group_entries_ = 0;
+        return;
+    }
+    for (size_t i = 1; i < group_classes_.size() && i <= 4; ++i)
+        if (!class_stream_[i - 1]) {
+            int lo = 0;
+            NAER_CK(cudaStreamGetPriority(stream_, &lo));
+            NAER_CK(cudaStreamCreateWithPriority(&class_stream_[i - 1], cudaStreamNonBlocking, lo));
+        }
+    for (auto& e : class_event_)
+        if (!e && group_classes_.size() > 1) NAER_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+}
+
+template <bool kGrid>
+static const void* group_kernel_of(uint32_t per, bool stdp) {
+    if (per == 4) return stdp ? (const void*)k_group<kGrid, 4, true> : (const void*)k_group<kGrid, 4, false>;
+    return stdp ? (const void*)k_group<kGrid, 1, true> : (const void*)k_group<kGrid, 1, false>;
+}
+const void* Engine::group_kernel(const GroupClass& c) const {
+    return group_form_ == kGroupGrid ? group_kernel_of<true>(c.per, c.stdp) : group_kernel_of<false>(c.per, c.stdp);
 }
 
 void Engine::launch_group(uint32_t steps, bool from_ctl) {
@@ -1150,31 +1335,61 @@ void Engine::launch_group(uint32_t steps, bool from_ctl) {
     if (grid) NAER_CK(cudaMemsetAsync(&d_ctl_->bar_arrive, 0, 8, stream_));
     const bool timed = profiling_ && !from_ctl;
     if (timed) NAER_CK(cudaEventRecord(timer_event(), stream_));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(group_blocks_);
-    cfg.blockDim = dim3(kGroupThreads);
-    cfg.dynamicSmemBytes = group_smem_;
-    cfg.stream = stream_;
-    cudaLaunchAttribute attr[1];
-    if (grid) {
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-    } else {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = group_blocks_;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    // the classes run beside one another: the first on the engine's stream,
+    // the others on streams forked from it and joined again
+    const size_t classes = group_classes_.size();
+    if (classes > 1) NAER_CK(cudaEventRecord(class_event_[0], stream_));
+    uint32_t first = 0, part = 0;
+    for (size_t i = 0; i < classes; ++i) {
+        const GroupClass& c = group_classes_[i];
+        const size_t lane = i == 0 ? 0 : (i - 1) % 4 + 1;  // a fifth class and on follow the earlier ones
+        cudaStream_t st = lane == 0 ? stream_ : class_stream_[lane - 1];
+        if (lane && i <= 4) NAER_CK(cudaStreamWaitEvent(st, class_event_[0], 0));
+        EngineDev e = eng_;
+        e.group_size = c.size;
+        e.group_order = d_gorder_ + first;
+        e.group_part = part;
+        e.group_own = c.own;
+        e.group_rows = c.rows ? 1u : 0u;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(c.nets * c.size);
+        cfg.blockDim = dim3(kGroupThreads);
+        cfg.dynamicSmemBytes = c.smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        if (grid) {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = c.size;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        }
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        void* args[3] = {&e, &s0, &steps};
+        NAER_CK(cudaLaunchKernelExC(&cfg, group_kernel(c), args));
+        first += c.nets;
+        part += c.nets * c.size;
     }
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    void* args[3] = {&eng_, &s0, &steps};
-    NAER_CK(cudaLaunchKernelExC(&cfg, group_kernel(grid), args));
+    for (size_t lane = 1; lane < classes && lane <= 4; ++lane) {
+        NAER_CK(cudaEventRecord(class_event_[lane], class_stream_[lane - 1]));
+        NAER_CK(cudaStreamWaitEvent(stream_, class_event_[lane], 0));
+    }
+    const bool several = eng_.n_nets > 1;
+    if (several) {
+        const uint64_t warps = eng_.record ? (uint64_t)steps * eng_.group_seg_n : 1u;
+        const uint32_t blocks = (uint32_t)std::min<uint64_t>((warps * 32 + kRasterThreads - 1) / kRasterThreads,
+                                                             (uint64_t)sm_count_ * 8);
+        k_raster<<<blocks, kRasterThreads, 0, stream_>>>(eng_, s0, steps);
+    }
     NAER_CK(cudaGetLastError());
     if (timed) {
         NAER_CK(cudaEventRecord(timer_event(), stream_));
         timer_kinds_.push_back(1);
     }
     if (!from_ctl) {
-        ++launches_;
+        launches_ += several ? 2 : 1;  // the classes' clusters count as one launch
         host_step_ += steps;
     }
 }
@@ -1465,7 +1680,7 @@ uint64_t Engine::run_graph(uint64_t nsteps, uint32_t graph_launches) {
     while (graph_exec_ && nsteps - done >= per) {
         NAER_CK(cudaGraphLaunch(graph_exec_, stream_));
         host_step_ += per;
-        launches_ += (group_active() ? 1ull : 2ull) * graph_launches;
+        launches_ += (group_active() && eng_.n_nets == 1 ? 1ull : 2ull) * graph_launches;
         done += per;
     }
     run(nsteps - done);

@@ -228,8 +228,21 @@ public:
 private:
     void build_arrays(NetHost& n);
     std::vector<std::pair<void*, size_t>>* alloc_log_ = nullptr;  // allocations of a build in progress
+    // Networks launched together: clusters of one size (or the grid).
+    struct GroupClass {
+        uint32_t size = 0;    // blocks of a cluster (of the grid)
+        uint32_t nets = 0;
+        uint32_t per = 1;     // neurons a lane
+        uint32_t own = 0;     // neurons of a block, at most
+        bool rows = false;    // row bounds in shared memory
+        bool stdp = false;
+        size_t smem = 0;
+    };
     void plan_group(const std::vector<PopDev>& pops);
-    const void* group_kernel(bool grid) const;
+    bool plan_one(const std::vector<PopDev>& pops);
+    bool plan_several(const std::vector<PopDev>& pops);
+    bool fit_class(GroupClass& c);
+    const void* group_kernel(const GroupClass& c) const;
     bool group_active() const { return group_form_ == kGroupGrid || (group_form_ == kGroupCluster && bar_skew_ == 0); }
     void launch_group(uint32_t steps, bool from_ctl);
     void launch_run(uint32_t steps);
@@ -298,13 +311,17 @@ private:
     // k_group: which form the installed networks step on, its geometry and tables
     static constexpr uint32_t kGroupNone = 0, kGroupCluster = 1, kGroupGrid = 2;
     uint32_t group_form_ = kGroupNone;
-    uint32_t group_per_ = 1;       // neurons a lane
-    uint32_t group_blocks_ = 0;    // blocks of the launch
-    size_t group_smem_ = 0;
+    std::vector<GroupClass> group_classes_;
+    uint32_t group_blocks_ = 0;    // blocks of all classes
+    cudaStream_t class_stream_[4] = {nullptr, nullptr, nullptr, nullptr};  // classes past the first run beside it
+    cudaEvent_t class_event_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     uint64_t group_entries_ = 0;   // spike records of all blocks
     uint64_t bar_skew_ = 0;
     std::vector<GroupChunk> h_chunks_;
     std::vector<GroupSeg> h_segs_;
+    std::vector<uint32_t> h_order_;  // networks, class by class, the most expensive first
+    uint32_t* d_gorder_ = nullptr;
+    size_t gorder_bytes_ = 0;
     GroupSeg* d_gsegs_ = nullptr;
     uint32_t* d_gtot_ = nullptr;
     size_t gsegs_bytes_ = 0, gtot_bytes_ = 0;

@@ -49,6 +49,7 @@ constexpr uint32_t kGroupMaxBlocks = 160; // blocks of a group, at most
 constexpr uint32_t kGroupPops = 8;        // populations of a network, at most
 constexpr uint32_t kGroupList = 1024;     // spikes of a window a block keeps in shared memory
 constexpr uint32_t kGroupSeg = 64;        // chunks of a raster segment
+constexpr uint32_t kRasterThreads = 256;
 constexpr uint32_t kGcLif = 1u << 16, kGcDrawn = 1u << 17;  // GroupChunk::info: LIF neurons; Poisson counts are drawn
 
 struct PopDev {
@@ -79,10 +80,13 @@ struct GroupChunk {
     uint32_t info;   // index among the network's populations | neurons (1..128) << 8 | kGcLif, kGcDrawn
 };
 
-// Up to kGroupSeg consecutive chunks: the piece of the raster one warp writes.
+// Up to kGroupSeg consecutive chunks of one network: the piece of the raster
+// one warp writes.
 struct GroupSeg {
-    uint32_t first;      // first chunk
+    uint32_t first;      // first chunk (of all networks')
     uint32_t count;
+    uint32_t word;       // first word of the spike bits
+    uint32_t per;        // words a chunk: neurons a lane, 1 or 4
     uint32_t pop_first;  // the network's first population
 };
 
@@ -137,10 +141,15 @@ struct NetDev {
     uint32_t window;        // steps per window: the smallest delay (1 with plasticity on), <= kGroupMaxWindow
     uint32_t pop_first;     // the network's populations: EngineDev::pops [pop_first, pop_first + pop_count)
     uint32_t pop_count;
-    uint32_t g_chunks;      // entries of EngineDev::group_chunks
+    uint32_t g_first;       // its chunks: EngineDev::group_chunks [g_first, g_first + g_chunks)
+    uint32_t g_chunks;
+    uint32_t seg_first;     // its raster segments: EngineDev::group_segs [seg_first, seg_first + seg_n)
+    uint32_t seg_n;
+    uint32_t g_word;        // its first word of EngineDev::group_bits
     uint32_t max_row;       // longest padded row
     uint32_t local;         // 1: a block delivers the spikes of its own neurons (window 1, no plasticity)
-    uint32_t pad_;
+    uint32_t q_cap;         // spike records of one of its blocks in a window, at most
+    uint64_t q_off;         // its blocks' records in EngineDev::queue[0] / qrow[0]
 };
 
 struct ChunkDev {
@@ -185,6 +194,8 @@ struct Ctl {
     unsigned int qtail[4];          // k_step: spikes queued in step s, slot s & 3 (zeroed with bar_arrive)
     unsigned int error;
     unsigned int pad_;
+    unsigned int raster_done;       // k_raster: blocks that have finished
+    unsigned int pad3_;
     unsigned int chk_code;          // NAER_CHECKED build: first out-of-bounds access (CheckCode), 0 = none
     unsigned int pad2_;
     unsigned long long chk_index;   // its index
@@ -231,19 +242,20 @@ struct EngineDev {
     uint32_t split_rest;
     uint32_t queue_cap;             // entries of queue[i] / qid[i]
     uint32_t bins;                  // k_step: shared-memory binning table entries (power of 2), 0 = off
-    // k_group
-    const GroupChunk* group_chunks; // the network's chunks, in storage order
+    // k_group / k_raster
+    const GroupChunk* group_chunks; // every network's chunks, in storage order
+    const uint32_t* group_order;    // several networks: those of this launch's clusters, the most expensive first
+    uint32_t group_size;            // blocks per cluster
+    uint32_t group_part;            // first block's entry of ev_part / ovf_part
     uint32_t* group_cnt;            // grid form: spikes of each block in the window
-    uint32_t* group_bits;           // [steps][group_words][neurons a lane] spikes of the launch: word k of a chunk =
-                                    // neuron k of each lane
-    const GroupSeg* group_segs;     // its raster segments, in address order
+    uint32_t* group_bits;           // [steps][group_words] spikes of the launch: word k of a chunk = neuron k of each lane
+    const GroupSeg* group_segs;     // raster segments of all networks, in address order
     uint32_t* group_q;              // [steps][group_seg_n] spikes per step and segment (0 between launches)
     uint32_t* group_tot;            // [steps] spikes per step (0 between launches)
     uint32_t group_seg_n;
-    uint32_t group_words;           // its chunks
+    uint32_t group_words;           // words of one step, all networks
     uint32_t group_rows;            // 1: the blocks keep their neurons' row bounds in shared memory
     uint32_t group_own;             // neurons of a block, at most (a multiple of 32)
-    uint32_t group_cap;             // spike records of a block in one window, at most
 };
 
 }  // namespace naer

@@ -1,12 +1,15 @@
-// k_group: the step kernel of one network without per-step launches of its
-// own for Poisson draws, with fewer barriers than k_step.  Included once, by
-// sim_kernels.cu, after the delivery helpers.
+// k_group: a step kernel without per-step launches of its own for Poisson
+// draws, with fewer barriers than k_step.  Included once, by sim_kernels.cu,
+// after the delivery helpers.
 //
 // Two forms share the code:
-//   kGrid = false  the network is stepped by one thread-block cluster,
-//                  synchronised by hardware cluster barriers (small networks)
-//   kGrid = true   by the whole (cooperative) grid, synchronised by the bounded
-//                  grid barrier
+//   kGrid = false  a network is stepped by one thread-block cluster,
+//                  synchronised by hardware cluster barriers.  Networks do not
+//                  interact, so each goes through all the steps of the launch
+//                  by itself; the clusters of a launch have one size, larger
+//                  networks are launched with larger clusters (Engine::plan_several)
+//   kGrid = true   one network is stepped by the whole (cooperative) grid,
+//                  synchronised by the bounded grid barrier
 // kPer neurons a lane (1 or 4): a warp's time over its neurons is a chain of
 // instructions, so networks with few neurons per warp take 1, the others 4
 // (vector loads, fewer instructions per neuron).
@@ -17,6 +20,9 @@
 // potential in registers and no synchronisation; then the group's spikes of
 // the window are delivered together.  Two barriers per window instead of two
 // per step, and only one where a block delivers its own spikes (NetDev::local).
+//
+// kPlastic: with the plasticity code; without it the kernel is shorter, and a
+// step passes once through most of its instructions.
 //
 // Of a block's warps, kGroupSteppers step neurons and deliver; the others draw
 // the Poisson counts of later steps meanwhile.
@@ -289,72 +295,75 @@ __device__ __forceinline__ void group_row(const NetDev& np, uint32_t slot, float
 // Raster of a launch.  Spikes are left as one bit per neuron (word u of a
 // chunk: neuron u of each lane).  raster_count: spikes of step k in segment
 // g, by one warp.
-template <int kPer>
+__device__ __forceinline__ uint4 raster_bits(const EngineDev& eng, const GroupSeg& seg, uint32_t k, uint32_t x) {
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    if (x < seg.count) {
+        const uint32_t* bits = eng.group_bits + (size_t)k * eng.group_words + seg.word;
+        if (seg.per == 4) m = __ldcg(reinterpret_cast<const uint4*>(bits) + x);
+        else m.x = __ldcg(bits + x);
+    }
+    return m;
+}
+
 __device__ __forceinline__ void raster_count(const EngineDev& eng, uint32_t k, uint32_t g, uint32_t lane) {
     const GroupSeg seg = eng.group_segs[g];
-    const uint32_t* bits = eng.group_bits + ((size_t)k * eng.group_words + seg.first) * kPer;
     uint32_t n = 0;
-#pragma unroll
-    for (uint32_t u = 0; u < kGroupSeg; u += 32)
-        if (u + lane < seg.count) {
-            if constexpr (kPer == 4) {
-                const uint4 m = __ldcg(reinterpret_cast<const uint4*>(bits) + u + lane);
-                n += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
-            } else {
-                n += __popc(__ldcg(bits + u + lane));
-            }
-        }
-    n = __reduce_add_sync(0xFFFFFFFFu, n);
-    if (lane == 0 && n) {
-        __stcg(eng.group_q + (size_t)k * eng.group_seg_n + g, n);
-        atomicAdd(eng.group_tot + k, n);
+    for (uint32_t u = lane; u < seg.count; u += 32) {
+        const uint4 m = raster_bits(eng, seg, k, u);
+        n += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
     }
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    if (lane != 0 || n == 0) return;
+    if (eng.group_seg_n == 1) {
+        __stcg(eng.group_tot + k, n);
+        return;
+    }
+    __stcg(eng.group_q + (size_t)k * eng.group_seg_n + g, n);
+    atomicAdd(eng.group_tot + k, n);
 }
 
 // Records of segment g in step k, by one warp: in step order and within a
 // step in ascending address.  Their place follows from the spikes of the
 // earlier steps and of the step's earlier segments.
-template <int kPer>
 __device__ __forceinline__ void raster_write(const EngineDev& eng, unsigned long long s0, uint32_t k, uint32_t g,
                                              unsigned long long rbase, uint32_t lane) {
+    // with one segment in all, the step's spikes are the segment's
     const uint32_t* q = eng.group_q + (size_t)k * eng.group_seg_n;
-    if (__ldcg(q + g) == 0) return;  // silent, or its network does not run in this step
+    unsigned long long before = 0;
+    const uint32_t mine = __ldcg(eng.group_seg_n > 1 ? q + g : eng.group_tot + k);
+    for (uint32_t x = lane; x < k; x += 32) before += __ldcg(eng.group_tot + x);
+    if (mine == 0) return;  // silent, or its network does not run in this step
+    for (uint32_t x = lane; x < g; x += 32) before += __ldcg(q + x);
     const GroupSeg seg = eng.group_segs[g];
-    const uint32_t* bits = eng.group_bits + ((size_t)k * eng.group_words + seg.first) * kPer;
     const GroupChunk* chunks = eng.group_chunks + seg.first;
     const PopDev* pops = eng.pops + seg.pop_first;
-    uint4 m[kGroupSeg / 32];
-#pragma unroll
-    for (uint32_t u = 0; u < kGroupSeg / 32; ++u) {
-        m[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (u * 32 + lane < seg.count) {
-            if constexpr (kPer == 4) m[u] = __ldcg(reinterpret_cast<const uint4*>(bits) + u * 32 + lane);
-            else m[u].x = __ldcg(bits + u * 32 + lane);
-        }
-    }
-    unsigned long long before = 0;
-    for (uint32_t x = lane; x < k; x += 32) before += __ldcg(eng.group_tot + x);
-    for (uint32_t x = lane; x < g; x += 32) before += __ldcg(q + x);
     unsigned long long at = rbase + warp_sum_u64(before);
+    constexpr uint32_t kTile = 2;
+    for (uint32_t u0 = lane; u0 - lane < seg.count; u0 += 32 * kTile) {
+        uint4 m[kTile];
 #pragma unroll
-    for (uint32_t u = 0; u < kGroupSeg / 32; ++u) {
-        const uint32_t c = __popc(m[u].x) + __popc(m[u].y) + __popc(m[u].z) + __popc(m[u].w);
-        if (!__any_sync(0xFFFFFFFFu, c != 0)) continue;
-        const uint32_t y = warp_scan(c, lane);
-        unsigned long long pos = at + (y - c);
-        at += __shfl_sync(0xFFFFFFFFu, y, 31);
-        if (!c) continue;
-        const GroupChunk ch = chunks[u * 32 + lane];
-        const PopDev& p = pops[ch.info & 0xFFu];
-        const uint32_t id0 = p.id_base + (ch.first - p.storage_base);
-        for (uint32_t lanes = m[u].x | m[u].y | m[u].z | m[u].w; lanes; lanes &= lanes - 1) {
-            const uint32_t l = __ffs(lanes) - 1;
+        for (uint32_t u = 0; u < kTile; ++u) m[u] = raster_bits(eng, seg, k, u0 + u * 32);
 #pragma unroll
-            for (uint32_t v = 0; v < (uint32_t)kPer; ++v)
-                if ((u4_get(m[u], v) >> l) & 1u) {
-                    if (pos < eng.raster_cap) __stcg(eng.raster + pos, make_uint2((uint32_t)(s0 + k), id0 + kPer * l + v));
-                    ++pos;
-                }
+        for (uint32_t u = 0; u < kTile; ++u) {
+            const uint32_t c = __popc(m[u].x) + __popc(m[u].y) + __popc(m[u].z) + __popc(m[u].w);
+            if (!__any_sync(0xFFFFFFFFu, c != 0)) continue;
+            const uint32_t y = warp_scan(c, lane);
+            unsigned long long pos = at + (y - c);
+            at += __shfl_sync(0xFFFFFFFFu, y, 31);
+            if (!c) continue;
+            const GroupChunk ch = chunks[u0 + u * 32];
+            const PopDev& p = pops[ch.info & 0xFFu];
+            const uint32_t id0 = p.id_base + (ch.first - p.storage_base);
+            for (uint32_t lanes = m[u].x | m[u].y | m[u].z | m[u].w; lanes; lanes &= lanes - 1) {
+                const uint32_t l = __ffs(lanes) - 1;
+#pragma unroll
+                for (uint32_t v = 0; v < 4; ++v)
+                    if ((u4_get(m[u], v) >> l) & 1u) {
+                        if (pos < eng.raster_cap)
+                            __stcg(eng.raster + pos, make_uint2((uint32_t)(s0 + k), id0 + seg.per * l + v));
+                        ++pos;
+                    }
+            }
         }
     }
 }
@@ -365,7 +374,8 @@ __device__ __forceinline__ void raster_end(const EngineDev& eng, unsigned long l
                                            unsigned long long rbase) {
     Ctl* ctl = eng.ctl;
     if (eng.record)
-        for (size_t x = threadIdx.x; x < (size_t)nsteps * eng.group_seg_n; x += blockDim.x) __stcg(eng.group_q + x, 0u);
+        for (size_t x = threadIdx.x; eng.group_seg_n > 1 && x < (size_t)nsteps * eng.group_seg_n; x += blockDim.x)
+            __stcg(eng.group_q + x, 0u);
     if (threadIdx.x < 32) {
         unsigned long long n = 0;
         if (eng.record)
@@ -383,11 +393,12 @@ __device__ __forceinline__ void raster_end(const EngineDev& eng, unsigned long l
                 ctl->raster_dropped += n - kept;
             }
             ctl->step = s0 + nsteps;
+            ctl->raster_done = 0;
         }
     }
 }
 
-template <bool kGrid, int kPer>
+template <bool kGrid, int kPer, bool kPlastic>
 __global__ void __launch_bounds__(kGroupThreads, 1)
     k_group(EngineDev eng, unsigned long long s0, uint32_t nsteps) {
     constexpr uint32_t kChunk = 32 * kPer;
@@ -396,7 +407,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ GroupShared sh;
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t csz = gridDim.x, rank = blockIdx.x;  // one cluster, or the grid
+    const uint32_t csz = kGrid ? gridDim.x : eng.group_size;  // blocks of the group
+    const uint32_t rank = kGrid ? blockIdx.x : blockIdx.x % csz, group = kGrid ? 0u : blockIdx.x / csz;
+    const bool several = !kGrid && eng.n_nets > 1;
     const bool drawer = wib >= kGroupSteppers;
     const uint32_t nwarps = csz * kGroupSteppers, gw = rank * kGroupSteppers + wib;  // stepping warps
     Ctl* ctl = eng.ctl;
@@ -408,15 +421,12 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     uint4* s_row = reinterpret_cast<uint4*>(sV + own_max);  // with eng.group_rows
     uint2* s_gc = reinterpret_cast<uint2*>(s_row + (eng.group_rows ? own_max : 0u));
     uint8_t* sR = reinterpret_cast<uint8_t*>(s_gc + own_max / kChunk);
-    // the block's spike records: in the grid form all of them, in the
-    // cluster form those past kGroupList
-    const size_t region = (size_t)blockIdx.x * eng.group_cap;
     unsigned long long bar_target = 0;
     unsigned long long ev = 0;
     uint32_t ovf = 0;
     if (s0 == kStepFromCtl) s0 = ctl->step;
     const unsigned long long rbase = ctl->raster_next;
-    const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
+    const bool timer = blockIdx.x == 0 && eng.group_part == 0 && threadIdx.x == 0;
     if (threadIdx.x == 0) {
         sh.bcfg = barrier_cfg(ctl);
         sh.ok = 1;
@@ -425,12 +435,16 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         for (int x = 0; x < 4; ++x) sh.ph[x] = 0;
     }
     bool ok = true;
+    const uint32_t ni = several ? eng.group_order[group] : 0u;
     static_assert(sizeof(NetDev) % 4 == 0 && sizeof(NetDev) / 4 <= kGroupThreads, "NetDev copied in words");
     if (threadIdx.x < sizeof(NetDev) / 4)
         reinterpret_cast<uint32_t*>(&sh.net)[threadIdx.x] =
-            __ldg(reinterpret_cast<const uint32_t*>(eng.nets) + threadIdx.x);
+            __ldg(reinterpret_cast<const uint32_t*>(eng.nets + ni) + threadIdx.x);
     __syncthreads();
     const NetDev& np = sh.net;
+    // the block's spike records: in the grid form all of them, in the cluster
+    // form those past kGroupList
+    const size_t region = np.q_off + (size_t)rank * np.q_cap;
     const unsigned long long a = s0 > np.start_step ? s0 : np.start_step;
     const unsigned long long b = s0 + nsteps < np.end_step ? s0 + nsteps : np.end_step;
     if (np.active && a < b) {
@@ -444,7 +458,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const uint32_t c = at / kGroupSteppers * nwarps + rank * kGroupSteppers + at % kGroupSteppers;
             uint2 gc = make_uint2(0u, 0u);
             if (c < np.g_chunks) {
-                const GroupChunk ch = eng.group_chunks[c];
+                const GroupChunk ch = eng.group_chunks[np.g_first + c];
                 gc = make_uint2(ch.first, ch.info);
             }
             s_gc[at] = gc;
@@ -500,10 +514,10 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const uint32_t w = (uint32_t)(b - s < W ? b - s : W);
             const uint32_t tl = (uint32_t)(s - np.start_step);
             uint32_t* bits =
-                eng.record ? eng.group_bits + (size_t)(s - s0) * eng.group_words * kPer : nullptr;
+                eng.record ? eng.group_bits + (size_t)(s - s0) * eng.group_words + np.g_word : nullptr;
             // spikes of one step of a chunk as bits for the raster
             auto put_bits = [&](uint32_t hit, uint32_t k, uint32_t chunk) {
-                uint32_t* to = bits + ((size_t)k * eng.group_words + chunk) * kPer;
+                uint32_t* to = bits + (size_t)k * eng.group_words + chunk * kPer;
                 if constexpr (kPer == 4) {
                     uint32_t m[4];
 #pragma unroll
@@ -679,12 +693,12 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const uint32_t mine = sh.n_spikes[par];
             if (!local) {
                 if (kGrid && threadIdx.x == 0) __stcg(eng.group_cnt + rank, mine);
-                if (!drawer && (kGrid || np.stdp_on)) {
+                if (!drawer && (kGrid || (kPlastic && np.stdp_on))) {
                     for (uint32_t e = threadIdx.x; e < mine; e += kGroupStepThreads) {
                         int4 head;
                         if (e < kGroupList) head = *reinterpret_cast<const int4*>(s_list + e);
                         else head = __ldcg(reinterpret_cast<const int4*>(eng.queue[0] + region + e));
-                        if (np.stdp_on && (uint32_t)head.x < np.n_plastic) {
+                        if (kPlastic && np.stdp_on && (uint32_t)head.x < np.n_plastic) {
                             float aux1;
                             stdp_post_spike(&sh.net, (uint32_t)head.x, (int32_t)tl + head.y, head.z, aux1);
                             head.w = __float_as_int(aux1);
@@ -746,7 +760,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 // still leaves every worker at most one
                 const uint32_t workers = local ? kGroupSteppers : nwarps;
                 const uint32_t narrow = (np.max_row + kPlasticPiece - 1) / kPlasticPiece;
-                const bool wide = !np.stdp_on && Q * narrow > workers;
+                const bool stdp = kPlastic && np.stdp_on;
+                const bool wide = !stdp && Q * narrow > workers;
                 const uint32_t pieces = wide ? (np.max_row + 127) / 128 : narrow;
                 const uint32_t want = (2u * workers + Q - 1) / Q;
                 const uint32_t split = want < pieces ? want : (pieces ? pieces : 1u);
@@ -773,20 +788,19 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         head = cluster_ld4(at);
                         row = cluster_ld4(at + 16);
                     } else {
-                        const size_t at = (size_t)reg * eng.group_cap + x;
+                        const size_t at = np.q_off + (size_t)reg * np.q_cap + x;
                         head = __ldcg(reinterpret_cast<const uint4*>(eng.queue[0] + at));
                         row = __ldcg(eng.qrow[0] + at);
                     }
                     if (!NAER_IN_BOUNDS(ctl, head.x, Ns, kChkQueue)) continue;
                     const uint64_t beg = ((uint64_t)row.y << 32) | row.x;
-                    if (np.stdp_on && head.x < np.n_plastic) {
+                    if (stdp && head.x < np.n_plastic) {
                         SpikeRec rec;
                         rec.net = 0;
                         rec.src = head.x;
                         rec.aux0 = (int32_t)head.z;
                         rec.aux1 = __uint_as_float(head.w);
-                        deliver_span(&sh.net, tl + head.y, rec, beg, beg + row.w, piece, split, kPlasticPiece, lane,
-                                     ev, ovf, ctl, bt);
+                        deliver_span(&sh.net, tl, rec, beg, beg + row.w, piece, split, kPlasticPiece, lane, ev, ovf, ctl, bt);
                     } else {
                         const float mult = (int32_t)head.z > 1 ? (float)(int32_t)head.z : 1.0f;
                         const uint32_t slot = ring_slot(tmod, head.y, D);
@@ -826,22 +840,22 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         // spikes per (step, segment); the last window's barrier made every
         // block's bits visible
         if (eng.record && ok) {
-            const uint32_t segs = eng.group_seg_n, items = (uint32_t)(b - a) * segs;
+            const uint32_t segs = np.seg_n, items = (uint32_t)(b - a) * segs;
             for (uint32_t it = rank * kGroupWarps + wib; it < items; it += csz * kGroupWarps)
-                raster_count<kPer>(eng, (uint32_t)(a - s0) + it / segs, it % segs, lane);
+                raster_count(eng, (uint32_t)(a - s0) + it / segs, np.seg_first + it % segs, lane);
         }
     }
-    if (ok) {
+    if (ok && !several) {
         if (eng.record) {
-            ok = group_barrier<kGrid>(ctl, bar_target, sh);  // the counts of every step
+            ok = group_barrier<kGrid>(ctl, bar_target, sh);  // the counts
             const uint32_t items = nsteps * eng.group_seg_n;
             for (uint32_t it = rank * kGroupWarps + wib; ok && it < items; it += csz * kGroupWarps)
-                raster_write<kPer>(eng, s0, it / eng.group_seg_n, it % eng.group_seg_n, rbase, lane);
+                raster_write(eng, s0, it / eng.group_seg_n, it % eng.group_seg_n, rbase, lane);
         }
         if (ok) ok = group_barrier<kGrid>(ctl, bar_target, sh);  // counts read before they are cleared
         if (ok && rank == 0) raster_end(eng, s0, nsteps, rbase);
     }
-    finish_counters(eng, ev, ovf, lane, &sh.ev, &sh.ovf);
+    finish_counters(eng, ev, ovf, lane, &sh.ev, &sh.ovf, eng.group_part);
     if (timer) {
         ctl->prof_phase_ns[0] += sh.ph[0];
         ctl->prof_phase_ns[1] += sh.ph[1];
@@ -853,9 +867,37 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     }
 }
 
-template __global__ void k_group<true, 1>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<true, 4>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<false, 1>(EngineDev, unsigned long long, uint32_t);
+// Raster of a launch over several networks (of one network, its group writes
+// the raster itself): warp by warp over (step, segment); the last block to
+// finish ends the launch.
+__global__ void __launch_bounds__(kRasterThreads) k_raster(EngineDev eng, unsigned long long s0, uint32_t nsteps) {
+    __shared__ bool s_last;
+    Ctl* ctl = eng.ctl;
+    if (s0 == kStepFromCtl) s0 = ctl->step;
+    const unsigned long long rbase = ctl->raster_next;
+    const uint32_t items = eng.record ? nsteps * eng.group_seg_n : 0u;
+    for (uint32_t it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += (gridDim.x * blockDim.x) >> 5)
+        raster_write(eng, s0, it / eng.group_seg_n, it % eng.group_seg_n, rbase, threadIdx.x & 31u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&ctl->raster_done, 1u) + 1 == gridDim.x;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    raster_end(eng, s0, nsteps, rbase);
+}
+
+
+template __global__ void k_group<true, 1, true>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<true, 1, false>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<true, 4, true>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<true, 4, false>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<false, 1, true>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<false, 1, false>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<false, 4, true>(EngineDev, unsigned long long, uint32_t);
+template __global__ void k_group<false, 4, false>(EngineDev, unsigned long long, uint32_t);
 
 size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows) {
     return kGroupList * sizeof(GroupSpike) + kGroupWarps * kGroupQueue * sizeof(DriveWindow) +

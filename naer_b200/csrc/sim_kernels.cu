@@ -1195,7 +1195,8 @@ __device__ __forceinline__ void store_chunk_state(uint32_t own, const ChunkCache
 // Per-thread event and history-overflow counts into the block's counters
 // (no same-address global atomics on the hot path).
 __device__ __forceinline__ void finish_counters(const EngineDev& eng, unsigned long long ev, uint32_t ovf,
-                                                uint32_t lane, unsigned long long* s_ev, uint32_t* s_ovf) {
+                                                uint32_t lane, unsigned long long* s_ev, uint32_t* s_ovf,
+                                                uint32_t part = 0) {
     ev = warp_sum_u64(ev);
     const unsigned long long ov = warp_sum_u64((unsigned long long)ovf);
     if (lane == 0) {
@@ -1204,8 +1205,8 @@ __device__ __forceinline__ void finish_counters(const EngineDev& eng, unsigned l
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (*s_ev) eng.ev_part[blockIdx.x] += *s_ev;
-        if (*s_ovf) eng.ovf_part[blockIdx.x] += *s_ovf;
+        if (*s_ev) eng.ev_part[part + blockIdx.x] += *s_ev;
+        if (*s_ovf) eng.ovf_part[part + blockIdx.x] += *s_ovf;
     }
 }
 

@@ -219,9 +219,11 @@ size_t step_smem_bytes(uint32_t own_max, bool smem_state, uint32_t bins = 0);
 __host__ __device__ inline size_t step_smem_offset(uint32_t bins) {
     return 16 + ((((size_t)bins * 12) + 15) & ~(size_t)15);
 }
-// one network stepped by a cluster or the grid in windows, kPer neurons a lane (group_kernel.cuh)
-template <bool kGrid, int kPer>
+// networks stepped in windows, each by a cluster, or one by the grid; kPer neurons a lane (group_kernel.cuh)
+template <bool kGrid, int kPer, bool kPlastic>
 __global__ void k_group(EngineDev eng, unsigned long long s0, uint32_t nsteps);
+// raster of a k_group launch over several networks
+__global__ void k_raster(EngineDev eng, unsigned long long s0, uint32_t nsteps);
 // dynamic shared memory of k_group for own_neurons neurons a block; rows: with their row bounds
 size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows);
 // Poisson counts of up to kDriveSlots steps ahead

@@ -13,6 +13,7 @@ import pytest
 
 from naer_b200 import _capi as capi
 from naer_b200 import spec as S
+from naer_b200.forms import Batch
 
 pytestmark = pytest.mark.gpu
 
@@ -185,3 +186,41 @@ def test_grid_wait_runs_out(lib):
         assert lib.naer_net_step(net.handle, 1) == capi.NAER_E_STATE
     finally:
         net.close()
+
+
+def uneven_members():
+    """Cluster sizes of 1 to 8 blocks, one and four neurons a lane, static and
+    plastic, windows of one and of many steps."""
+    ms = [S.plastic_indegree(n=n, k=k, seed=i, drive_rate_hz=30.0, stdp=i % 2 == 0).with_(exact=True)
+          for i, (n, k) in enumerate([(600, 40), (1601, 90), (5003, 150), (2222, 300), (9001, 200), (800, 60), (3100, 25),
+                                      (12000, 100), (1000, 500), (450, 20)])]
+    ms += [mixed_net(n, 12, dmin, dmax, sources=src, seed=40 + n, exact=True)
+           for n, dmin, dmax, src in [(700, 15, 15, 90), (2500, 3, 30, 0), (6500, 7, 9, 260)]]
+    return ms
+
+
+@pytest.mark.parametrize("record", [True, False])
+def test_batch_members_as_alone(lib, record):
+    ms = uneven_members()
+    runs = [64, 7, 130]
+    with Batch(ms, exact=True, raster_capacity=1 << 22 if record else 1).compile() as b:
+        l0 = b.stats()["kernel_launches"]
+        for c in runs:
+            b.run(c)
+        b.finish()
+        assert b.stats()["kernel_launches"] - l0 == 2 * sum((c + 63) // 64 for c in runs)
+        spikes = b.read_spikes()
+        states = [b.read_state(i, m.neurons) for i, m in enumerate(ms)]
+    if record:
+        assert np.all(np.diff(spikes[1].astype(np.int64)) >= 0)  # step by step
+    for i, m in enumerate(ms):
+        with S.build(m) as net:
+            net.run(sum(runs))
+            net.finish()
+            st, ids = net.read_spikes()
+            v, r = net.read_state()
+        assert np.array_equal(states[i][0].view(np.uint32), v.view(np.uint32)), i
+        assert np.array_equal(states[i][1], r), i
+        if record:
+            bst, bids = b.member_spikes(i, spikes)
+            assert len(ids) > 5 and np.array_equal(bst, st) and np.array_equal(bids, ids), i
