@@ -990,7 +990,7 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     eng_.ev_part = d_ev_part_;
     eng_.ovf_part = d_ovf_part_;
     if (group_form_ != kGroupNone) {
-        const uint64_t steps = tuning_.launch_steps;
+        const uint64_t steps = group_launch_steps();
         regrow(reinterpret_cast<void*&>(d_gcnt_), gcnt_bytes_, group_blocks_ * 4ull);
         NAER_CK(cudaMemsetAsync(&d_ctl_->raster_done, 0, 4, stream_));
         if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * eng_.group_words * 4ull);
@@ -1208,7 +1208,8 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
     std::sort(targets.begin(), targets.end());
     double best = 1e30;
     std::vector<int> pick(count), best_pick;
-    for (size_t x = 0; x < targets.size(); x += std::max<size_t>(1, targets.size() / 64)) {
+    const size_t tries = count > 128 ? 16 : 64;
+    for (size_t x = 0; x < targets.size(); x += std::max<size_t>(1, targets.size() / tries)) {
         for (size_t i = 0; i < count; ++i) {
             int k = 0;
             while (k + 1 < kSizes && t[i * kSizes + k] > targets[x]) ++k;
@@ -1625,7 +1626,7 @@ void Engine::run_launches(uint64_t nsteps) {
     // Poisson counts of a chunk of steps are drawn first (full occupancy),
     // then the persistent kernel simulates the chunk
     while (nsteps > 0) {
-        const uint32_t n = (uint32_t)std::min<uint64_t>(nsteps, tuning_.launch_steps);
+        const uint32_t n = (uint32_t)std::min<uint64_t>(nsteps, group_active() ? group_launch_steps() : tuning_.launch_steps);
         if (group_active()) {
             launch_group(n, false);
         } else {

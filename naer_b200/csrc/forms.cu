@@ -408,6 +408,11 @@ void Server::loop() {
         tn.launch_steps = prm_.launch_steps;
         tn.blocks_per_sm = prm_.blocks_per_sm;
         tn.step_kernel = prm_.step_kernel;
+        // jobs in clusters of their own leave the builder SMs to run on, and a
+        // launch costs as much as two or three steps (24 jobs of up to 20k
+        // neurons, all at once, ms until the last: 35.0 with 16 steps a launch,
+        // 33.8 with 32, 33.0 with 64; 78.6 on the two-barrier kernel)
+        tn.group_steps = std::max<uint32_t>(32, prm_.launch_steps);
         eng->set_tuning(tn);
         // Admission keeps the running set within the step kernel's fastest
         // geometry (neuron state in shared memory, most blocks per SM).  A
