@@ -853,6 +853,7 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
         for (const ConnSpec& c : n.conns)
             if (n.pops[c.src].size && n.pops[c.dst].size) d.window = std::min(d.window, c.spec.delay_min);
         if (d.stdp_on) d.window = 1;  // a weight update sees the post-synaptic state of its own step
+        if (aggregation == NAER_AGG_DETERMINISTIC) d.window = 1;  // events are ordered step by step
         h_nets_.push_back(d);
         id_off += n.n_ids;
         if (id_off > 0xFFFFFFFFull) throw Error(NAER_E_OVERFLOW, "more than 2^32 neuron addresses in one engine");
@@ -1068,9 +1069,9 @@ bool Engine::fit_class(GroupClass& c) {
     NAER_CK(cudaFuncGetAttributes(&fa, kern));
     const int most = optin - (int)fa.sharedSizeBytes;
     NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    if (group_smem_bytes(c.own, c.per, false) > (size_t)most) return false;
-    c.rows = group_smem_bytes(c.own, c.per, true) <= (size_t)most;
-    c.smem = group_smem_bytes(c.own, c.per, c.rows);
+    if (group_smem_bytes(c.own, c.per, false, c.det) > (size_t)most) return false;
+    c.rows = group_smem_bytes(c.own, c.per, true, c.det) <= (size_t)most;
+    c.smem = group_smem_bytes(c.own, c.per, c.rows, c.det);
     if (group_form_ == kGroupGrid) return true;
     NAER_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
@@ -1103,6 +1104,12 @@ bool Engine::fit_class(GroupClass& c) {
 //   k_step from 500k neurons (700k / 300: 17.0, grid 17.0; 1M / 1000: 27.0,
 //     27.4) or 250k with plasticity (300k / 300: 14.1, 14.1), unless windows
 //     are longer than one step
+//   deterministic aggregation (windows of one step, k_det_step where not):
+//     the same lines, except that the grid pays up to 250k neurons (200k /
+//     1000: 20.2, k_det_step 23.2; 400k / 500: 23.7, 25.2, but 400k / 1000:
+//     32.1, 27.0: k_det_step has a third more warps to wait for the events'
+//     exchanges), with plasticity up to 600k (300k / 300: 24.4, 29.9; 600k /
+//     200: 34.0, 36.2)
 //   block-local delivery (one barrier a step) up to 500k synapses a block: a
 //     block's share of a step's spikes varies, which costs more than the
 //     barrier saves once it is bound by its reductions (50k / 400: 6.6 against
@@ -1110,6 +1117,7 @@ bool Engine::fit_class(GroupClass& c) {
 bool Engine::plan_one(const std::vector<PopDev>& pops) {
     NetDev& d = h_nets_[0];
     const NetHost& n = *nets_[0];
+    const bool det = aggregation_ == NAER_AGG_DETERMINISTIC;
     const uint32_t step_warps = kGroupStepThreads / 32, chunks = group_chunks(d, pops, 1);
     uint32_t c = 16;
     const bool cluster = chunks <= c * step_warps ||
@@ -1123,11 +1131,13 @@ bool Engine::plan_one(const std::vector<PopDev>& pops) {
     k.per = cluster || chunks <= 2 * c * step_warps ? 1 : 4;
     k.own = group_own(d, pops, c, k.per);
     k.stdp = d.stdp_on != 0;
+    k.det = det;
     // the windows' spike records (32 B each) stay below 256 MB
     const uint64_t most_entries = 8000000;
     if (!cluster && (uint64_t)c * k.own * d.window > most_entries)
         d.window = (uint32_t)std::max<uint64_t>(1, most_entries / ((uint64_t)c * k.own));
-    if (!cluster && d.window == 1 && n.n_storage > (d.stdp_on ? 250000u : 500000u)) return false;
+    if (!cluster && d.window == 1 && n.n_storage > (det ? d.stdp_on ? 600000u : 250000u : d.stdp_on ? 250000u : 500000u))
+        return false;
     if (!fit_class(k)) return false;
     group_classes_.assign(1, k);
     h_order_.assign(1, 0u);
@@ -1257,7 +1267,8 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
 void Engine::plan_group(const std::vector<PopDev>& pops) {
     group_form_ = kGroupNone;
     group_entries_ = 0;
-    if (aggregation_ == NAER_AGG_DETERMINISTIC || !tuning_.group_allowed() || h_nets_.empty()) return;
+    const bool det = aggregation_ == NAER_AGG_DETERMINISTIC;
+    if ((det && h_nets_.size() > 1) || !tuning_.group_allowed() || h_nets_.empty()) return;
     bool ok = true;
     for (const NetDev& d : h_nets_) ok = ok && d.pop_count > 0 && d.pop_count <= kGroupPops;
     ok = ok && (h_nets_.size() == 1 ? plan_one(pops) : plan_several(pops));
@@ -1294,7 +1305,7 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
                 h_segs_.push_back(GroupSeg{d.g_first + f, std::min(seg, d.g_chunks - f), words + f * c.per, c.per, d.pop_first});
             d.seg_n = (uint32_t)h_segs_.size() - d.seg_first;
             words += d.g_chunks * c.per;
-            d.local = d.window == 1 && !d.stdp_on && nets_[i]->synapses <= 500000ull * c.size ? 1u : 0u;
+            d.local = d.window == 1 && !d.stdp_on && !det && nets_[i]->synapses <= 500000ull * c.size ? 1u : 0u;
             d.q_cap = group_own(d, pops, c.size, c.per) * d.window;
             d.q_off = group_entries_;
             group_entries_ += (uint64_t)d.q_cap * c.size;
@@ -1321,13 +1332,15 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
         if (!e && group_classes_.size() > 1) NAER_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 }
 
-template <bool kGrid>
-static const void* group_kernel_of(uint32_t per, bool stdp) {
-    if (per == 4) return stdp ? (const void*)k_group<kGrid, 4, true> : (const void*)k_group<kGrid, 4, false>;
-    return stdp ? (const void*)k_group<kGrid, 1, true> : (const void*)k_group<kGrid, 1, false>;
+template <bool kGrid, int kPer>
+static const void* group_kernel_of(bool stdp, bool det) {
+    if (det) return stdp ? (const void*)k_group<kGrid, kPer, true, true> : (const void*)k_group<kGrid, kPer, false, true>;
+    return stdp ? (const void*)k_group<kGrid, kPer, true, false> : (const void*)k_group<kGrid, kPer, false, false>;
 }
 const void* Engine::group_kernel(const GroupClass& c) const {
-    return group_form_ == kGroupGrid ? group_kernel_of<true>(c.per, c.stdp) : group_kernel_of<false>(c.per, c.stdp);
+    if (group_form_ == kGroupGrid)
+        return c.per == 4 ? group_kernel_of<true, 4>(c.stdp, c.det) : group_kernel_of<true, 1>(c.stdp, c.det);
+    return c.per == 4 ? group_kernel_of<false, 4>(c.stdp, c.det) : group_kernel_of<false, 1>(c.stdp, c.det);
 }
 
 void Engine::launch_group(uint32_t steps, bool from_ctl) {

@@ -238,6 +238,7 @@ private:
         uint32_t own = 0;     // neurons of a block, at most
         bool rows = false;    // row bounds in shared memory
         bool stdp = false;
+        bool det = false;     // deterministic aggregation
         size_t smem = 0;
     };
     void plan_group(const std::vector<PopDev>& pops);

@@ -24,6 +24,9 @@
 // kPlastic: with the plasticity code; without it the kernel is shorter, and a
 // step passes once through most of its instructions.
 //
+// kDet: deterministic aggregation of one network, in windows of one step with
+// a third barrier (det_link, det_fold).
+//
 // Of a block's warps, kGroupSteppers step neurons and deliver; the others draw
 // the Poisson counts of later steps meanwhile.
 //
@@ -41,6 +44,7 @@ constexpr uint32_t kGroupWarps = kGroupThreads / 32;
 constexpr uint32_t kGroupSteppers = kGroupStepThreads / 32;
 constexpr uint32_t kGroupDrawers = kGroupWarps - kGroupSteppers;
 constexpr uint32_t kGroupAhead = 4;    // steps drawn ahead of the simulation, at least
+constexpr uint32_t kDetStarts = 384;   // list starts a warp keeps (deterministic aggregation)
 constexpr uint32_t kGroupQueue = 64;   // windows a warp can hold (31 left over + 32)
 static_assert(2 * kGroupMaxWindow <= kDriveSlots, "counts of two windows fit the drive ring");
 static_assert(4 * kGroupMaxWindow <= 64, "a lane's spikes of a window fit 64 bits");
@@ -398,7 +402,145 @@ __device__ __forceinline__ void raster_end(const EngineDev& eng, unsigned long l
     }
 }
 
-template <bool kGrid, int kPer, bool kPlastic>
+// Deterministic aggregation.  The order of a step's additions to a ring cell
+// is that of the synapse indices j (k_det_step): every event of the step
+// stores its weight at ev_w[j] and links itself into its cell's list, and
+// after a barrier the event that started a list folds it in ascending j and
+// adds the fold to the cell.  The warp that linked a list's first event keeps
+// {j, cell, weight} in its own part of shared memory (kDetStarts places), so
+// that the fold reads no row again: one load of the list's head, and for a
+// list of one event (most of them) nothing else.  A warp with more starts
+// than places goes over its rows a second time instead.
+// Bound by the same chain of latencies as the rest of k_group, with one
+// exchange and one head load more and the third barrier.  Per grid step,
+// against k_drive + k_det_step (whose fold reads the rows and links of all
+// events again, between barriers of two blocks an SM): 1k neurons /
+// out-degree 50: 6.0 against 10.5 us; 12k / 600: 12.5 against 17.9; 100k /
+// 500: 16.0 against 21.9; plastic 5k / 200: 8.4 against 21.4, 80k / 800: 14.7
+// against 27.7.
+struct __align__(16) DetStart {
+    uint32_t j, cell;
+    float w;
+    uint32_t pad;  // one 128-bit access
+};
+
+// Links one piece of a row (psz synapses, kBatch a lane at a time): all loads
+// of a batch before the first exchange, all exchanges before the first of
+// their results is used.  Returns the warp's starts (may exceed kDetStarts).
+template <int kBatch>
+__device__ __forceinline__ uint32_t det_link(const NetDev& np, uint32_t tl, uint32_t tmod, const uint4& spike,
+                                             uint64_t beg, uint32_t len, uint32_t piece, uint32_t split, DetStart* starts,
+                                             uint32_t n, uint32_t lane, unsigned long long& ev, uint32_t& ovf, Ctl* ctl) {
+    const uint32_t D = np.ring_slots, Ns = np.n_storage;
+    const uint32_t* __restrict__ tgt_a = np.tgt + beg;
+    const uint8_t* __restrict__ d_a = np.dly + beg;
+    float* w_a = np.w + beg;
+    float* __restrict__ ev_w = np.ev_w + beg;
+    uint32_t* __restrict__ ev_next = np.ev_next + beg;
+    uint32_t* __restrict__ heads = np.cell_head;
+    const bool plastic = np.stdp_on && spike.x < np.n_plastic;
+    const int32_t aux0 = (int32_t)spike.z;
+    const float mult = !plastic && aux0 > 1 ? (float)aux0 : 1.0f;
+    StdpView sv;
+    if (plastic) sv = stdp_view(np);
+    for (uint32_t off = piece * 32 * kBatch; off < len; off += split * 32 * kBatch) {
+        uint32_t cell[kBatch], tgt[kBatch], d[kBatch], old[kBatch];
+        float w[kBatch];
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u) {
+            const uint32_t x = off + 32 * u + lane;
+            tgt[u] = kTgtSentinel;
+            if (x < len && NAER_IN_BOUNDS(ctl, beg + x, np.syn_cap, kChkEventList)) {
+                tgt[u] = __ldcg(tgt_a + x);
+                d[u] = __ldcg(d_a + x);
+                w[u] = __ldcg(w_a + x);
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u) {
+            const bool on = tgt[u] != kTgtSentinel && NAER_IN_BOUNDS(ctl, tgt[u], Ns, kChkRing);
+            cell[u] = on ? ring_slot(tmod, d[u], D) * Ns + tgt[u] : kTgtSentinel;
+            if (!on) continue;
+            const uint32_t x = off + 32 * u + lane;
+            old[u] = atomicExch(heads + cell[u], (uint32_t)(beg + x));
+            if (plastic && tgt[u] < np.n_plastic) {
+                w[u] = stdp_update(sv, w[u], tgt[u], (int32_t)tl, aux0, __uint_as_float(spike.w), ovf);
+                __stcg(w_a + x, w[u]);
+            }
+            if (mult != 1.0f) w[u] = __fmul_rn(w[u], mult);
+            __stcg(ev_w + x, w[u]);
+            ++ev;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u) {
+            const bool on = cell[u] != kTgtSentinel;
+            const uint32_t x = off + 32 * u + lane;
+            if (on) __stcg(ev_next + x, old[u]);
+            const bool first = on && old[u] == kNoEvent;
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, first);
+            const uint32_t pos = n + __popc(bal & ((1u << lane) - 1u));
+            if (first && pos < kDetStarts) starts[pos] = DetStart{(uint32_t)beg + x, cell[u], w[u], 0u};
+            n += __popc(bal);
+        }
+    }
+    return n;
+}
+
+// Empties a list and adds its fold to the cell (j: its first event, of weight
+// w).  No other thread touches the list or the cell in this phase.
+__device__ __forceinline__ void det_add(const NetDev& np, uint32_t cell, uint32_t hd, uint32_t j, float w) {
+    __stcg(np.cell_head + cell, kNoEvent);
+    red_add_f32(np.ring + cell, hd == j ? w : fold_from_start(np.ev_w, np.ev_next, hd, j, w));
+}
+
+// The fold over a warp's starts, kFold a lane with their heads in flight.
+__device__ __forceinline__ void det_fold(const NetDev& np, const DetStart* starts, uint32_t n, uint32_t lane) {
+    constexpr uint32_t kFold = 4;
+    for (uint32_t x0 = lane; x0 < n; x0 += 32 * kFold) {
+        uint32_t hd[kFold];
+#pragma unroll
+        for (uint32_t u = 0; u < kFold; ++u)
+            if (x0 + 32 * u < n) hd[u] = __ldcg(np.cell_head + starts[x0 + 32 * u].cell);
+#pragma unroll
+        for (uint32_t u = 0; u < kFold; ++u)
+            if (x0 + 32 * u < n) {
+                const DetStart st = starts[x0 + 32 * u];
+                det_add(np, st.cell, hd[u], st.j, st.w);
+            }
+    }
+}
+
+// The fold over a piece of a row read again: its events without a next one.
+template <int kBatch>
+__device__ __forceinline__ void det_refold(const NetDev& np, uint32_t tmod, uint64_t beg, uint32_t len, uint32_t piece,
+                                           uint32_t split, uint32_t lane, Ctl* ctl) {
+    const uint32_t* __restrict__ tgt_a = np.tgt + beg;
+    const uint8_t* __restrict__ d_a = np.dly + beg;
+    for (uint32_t off = piece * 32 * kBatch; off < len; off += split * 32 * kBatch) {
+        uint32_t cell[kBatch], next[kBatch], hd[kBatch];
+        float w[kBatch];
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u) {
+            const uint32_t x = off + 32 * u + lane;
+            cell[u] = kTgtSentinel;
+            if (x >= len || !NAER_IN_BOUNDS(ctl, beg + x, np.syn_cap, kChkEventList)) continue;
+            const uint32_t tgt = __ldcg(tgt_a + x), d = __ldcg(d_a + x);
+            next[u] = __ldcg(np.ev_next + beg + x);
+            w[u] = __ldcg(np.ev_w + beg + x);
+            if (tgt != kTgtSentinel && NAER_IN_BOUNDS(ctl, tgt, np.n_storage, kChkRing))
+                cell[u] = ring_slot(tmod, d, np.ring_slots) * np.n_storage + tgt;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u)
+            if (cell[u] != kTgtSentinel && next[u] == kNoEvent) hd[u] = __ldcg(np.cell_head + cell[u]);
+#pragma unroll
+        for (uint32_t u = 0; u < (uint32_t)kBatch; ++u)
+            if (cell[u] != kTgtSentinel && next[u] == kNoEvent)
+                det_add(np, cell[u], hd[u], (uint32_t)(beg + off + 32 * u + lane), w[u]);
+    }
+}
+
+template <bool kGrid, int kPer, bool kPlastic, bool kDet>
 __global__ void __launch_bounds__(kGroupThreads, 1)
     k_group(EngineDev eng, unsigned long long s0, uint32_t nsteps) {
     constexpr uint32_t kChunk = 32 * kPer;
@@ -421,6 +563,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     uint4* s_row = reinterpret_cast<uint4*>(sV + own_max);  // with eng.group_rows
     uint2* s_gc = reinterpret_cast<uint2*>(s_row + (eng.group_rows ? own_max : 0u));
     uint8_t* sR = reinterpret_cast<uint8_t*>(s_gc + own_max / kChunk);
+    // deterministic aggregation: the warp's list starts
+    DetStart* starts = reinterpret_cast<DetStart*>(sR + own_max) + wib * kDetStarts;
     unsigned long long bar_target = 0;
     unsigned long long ev = 0;
     uint32_t ovf = 0;
@@ -506,7 +650,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         // block that found them delivers, as soon as its neurons have
         // stepped (ring slot s is read and cleared only in step s, and no
         // spike of step s lands in it): one barrier per step
-        const bool local = np.local;
+        const bool local = !kDet && np.local;
         uint32_t par = 0;  // window parity
         uint32_t tmod = (uint32_t)(a - np.start_step) % D;
         for (unsigned long long s = a; s < b; s += W, par ^= 1u) {
@@ -747,6 +891,33 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 }
             }
             // ---- 4. every row of the window's spikes
+            uint32_t workers = 0, split = 1, items = 0, n_starts = 0;
+            bool wide = false;
+            // spike e of the window: the block that holds it, and its place there
+            auto fetch = [&](uint32_t e, uint4& head, uint4& row) {
+                uint32_t reg = rank, x = e;
+                if (!local) {
+                    if (!kGrid) {
+                        reg = __popc(__ballot_sync(0xFFFFFFFFu, lane < csz && below <= e)) - 1u;
+                        x = e - __shfl_sync(0xFFFFFFFFu, below, reg);
+                    } else {
+                        reg = locate(sh.first, csz, e);
+                        x = e - sh.first[reg];
+                    }
+                }
+                if (local && x < kGroupList) {
+                    head = *reinterpret_cast<const uint4*>(s_list + x);
+                    row = s_list[x].row;
+                } else if (!kGrid && x < kGroupList) {
+                    const uint32_t at = cluster_map(s_list + x, reg);
+                    head = cluster_ld4(at);
+                    row = cluster_ld4(at + 16);
+                } else {
+                    const size_t at = np.q_off + (size_t)reg * np.q_cap + x;
+                    head = __ldcg(reinterpret_cast<const uint4*>(eng.queue[0] + at));
+                    row = __ldcg(eng.qrow[0] + at);
+                }
+            };
             if (drawer) {
                 // meanwhile: counts of the steps `ahead` of the next window
                 const unsigned long long goal = s + w + ahead < b ? s + w + ahead : b;
@@ -758,43 +929,25 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 // row pieces: enough items for the workers, no more than
                 // the longest row has; one synapse a lane where that
                 // still leaves every worker at most one
-                const uint32_t workers = local ? kGroupSteppers : nwarps;
+                workers = local ? kGroupSteppers : nwarps;
                 const uint32_t narrow = (np.max_row + kPlasticPiece - 1) / kPlasticPiece;
                 const bool stdp = kPlastic && np.stdp_on;
-                const bool wide = !stdp && Q * narrow > workers;
+                wide = (kDet || !stdp) && Q * narrow > workers;
                 const uint32_t pieces = wide ? (np.max_row + 127) / 128 : narrow;
                 const uint32_t want = (2u * workers + Q - 1) / Q;
-                const uint32_t split = want < pieces ? want : (pieces ? pieces : 1u);
-                const uint32_t items = Q * split;  // at most Q + 2 * workers
+                split = want < pieces ? want : (pieces ? pieces : 1u);
+                items = Q * split;  // at most Q + 2 * workers
                 BinTable bt{};
                 for (uint32_t it = local ? wib : gw; it < items; it += workers) {
                     const uint32_t e = it / split, piece = it - e * split;
-                    uint32_t reg = rank, x = e;  // the block that holds spike e, and the spike's place there
                     uint4 head, row;
-                    if (!local) {
-                        if (!kGrid) {
-                            reg = __popc(__ballot_sync(0xFFFFFFFFu, lane < csz && below <= e)) - 1u;
-                            x = e - __shfl_sync(0xFFFFFFFFu, below, reg);
-                        } else {
-                            reg = locate(sh.first, csz, e);
-                            x = e - sh.first[reg];
-                        }
-                    }
-                    if (local && x < kGroupList) {
-                        head = *reinterpret_cast<const uint4*>(s_list + x);
-                        row = s_list[x].row;
-                    } else if (!kGrid && x < kGroupList) {
-                        const uint32_t at = cluster_map(s_list + x, reg);
-                        head = cluster_ld4(at);
-                        row = cluster_ld4(at + 16);
-                    } else {
-                        const size_t at = np.q_off + (size_t)reg * np.q_cap + x;
-                        head = __ldcg(reinterpret_cast<const uint4*>(eng.queue[0] + at));
-                        row = __ldcg(eng.qrow[0] + at);
-                    }
+                    fetch(e, head, row);
                     if (!NAER_IN_BOUNDS(ctl, head.x, Ns, kChkQueue)) continue;
                     const uint64_t beg = ((uint64_t)row.y << 32) | row.x;
-                    if (stdp && head.x < np.n_plastic) {
+                    if constexpr (kDet) {
+                        n_starts = wide ? det_link<4>(np, tl, tmod, head, beg, row.w, piece, split, starts, n_starts, lane, ev, ovf, ctl)
+                                        : det_link<1>(np, tl, tmod, head, beg, row.w, piece, split, starts, n_starts, lane, ev, ovf, ctl);
+                    } else if (stdp && head.x < np.n_plastic) {
                         SpikeRec rec;
                         rec.net = 0;
                         rec.src = head.x;
@@ -806,6 +959,22 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         const uint32_t slot = ring_slot(tmod, head.y, D);
                         if (wide) group_row<true>(np, slot, mult, beg, row.w, piece, split, lane, ev, ctl);
                         else group_row<false>(np, slot, mult, beg, row.w, piece, split, lane, ev, ctl);
+                    }
+                }
+            }
+            if (kDet && Q) {  // every event is linked: fold
+                ok = group_barrier<kGrid>(ctl, bar_target, sh);
+                if (!ok) break;
+                if (!drawer && n_starts <= kDetStarts) {
+                    det_fold(np, starts, n_starts, lane);
+                } else if (!drawer) {
+                    for (uint32_t it = gw; it < items; it += workers) {
+                        const uint32_t e = it / split;
+                        uint4 head, row;
+                        fetch(e, head, row);
+                        const uint64_t beg = ((uint64_t)row.y << 32) | row.x;
+                        if (wide) det_refold<4>(np, tmod, beg, row.w, it - e * split, split, lane, ctl);
+                        else det_refold<1>(np, tmod, beg, row.w, it - e * split, split, lane, ctl);
                     }
                 }
             }
@@ -890,18 +1059,21 @@ __global__ void __launch_bounds__(kRasterThreads) k_raster(EngineDev eng, unsign
 }
 
 
-template __global__ void k_group<true, 1, true>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<true, 1, false>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<true, 4, true>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<true, 4, false>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<false, 1, true>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<false, 1, false>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<false, 4, true>(EngineDev, unsigned long long, uint32_t);
-template __global__ void k_group<false, 4, false>(EngineDev, unsigned long long, uint32_t);
+#define NAER_GROUP(grid, per)                                                                      \
+    template __global__ void k_group<grid, per, true, false>(EngineDev, unsigned long long, uint32_t);  \
+    template __global__ void k_group<grid, per, false, false>(EngineDev, unsigned long long, uint32_t); \
+    template __global__ void k_group<grid, per, true, true>(EngineDev, unsigned long long, uint32_t);   \
+    template __global__ void k_group<grid, per, false, true>(EngineDev, unsigned long long, uint32_t);
+NAER_GROUP(true, 1)
+NAER_GROUP(true, 4)
+NAER_GROUP(false, 1)
+NAER_GROUP(false, 4)
+#undef NAER_GROUP
 
-size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows) {
+size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows, bool det) {
     return kGroupList * sizeof(GroupSpike) + kGroupWarps * kGroupQueue * sizeof(DriveWindow) +
-           (size_t)own_neurons * (5 + (rows ? 16 : 0)) + own_neurons / (32 * per_lane) * sizeof(uint2);
+           (size_t)own_neurons * (5 + (rows ? 16 : 0)) + own_neurons / (32 * per_lane) * sizeof(uint2) +
+           (det ? kGroupSteppers * kDetStarts * sizeof(DetStart) : 0);
 }
 
 }  // namespace naer

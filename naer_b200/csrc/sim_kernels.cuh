@@ -219,13 +219,14 @@ size_t step_smem_bytes(uint32_t own_max, bool smem_state, uint32_t bins = 0);
 __host__ __device__ inline size_t step_smem_offset(uint32_t bins) {
     return 16 + ((((size_t)bins * 12) + 15) & ~(size_t)15);
 }
-// networks stepped in windows, each by a cluster, or one by the grid; kPer neurons a lane (group_kernel.cuh)
-template <bool kGrid, int kPer, bool kPlastic>
+// networks stepped in windows, each by a cluster, or one by the grid; kPer neurons a lane (group_kernel.cuh);
+// kDet: one network with deterministic aggregation
+template <bool kGrid, int kPer, bool kPlastic, bool kDet>
 __global__ void k_group(EngineDev eng, unsigned long long s0, uint32_t nsteps);
 // raster of a k_group launch over several networks
 __global__ void k_raster(EngineDev eng, unsigned long long s0, uint32_t nsteps);
 // dynamic shared memory of k_group for own_neurons neurons a block; rows: with their row bounds
-size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows);
+size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows, bool det = false);
 // Poisson counts of up to kDriveSlots steps ahead
 __global__ void k_drive(EngineDev eng, unsigned long long s_first, uint32_t nsteps);
 

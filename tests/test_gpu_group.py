@@ -111,6 +111,30 @@ def test_two_plastic_populations_and_odd_sizes(O):
     assert_matches(O, s, [500])
 
 
+@pytest.mark.parametrize("n,k,dmin,dmax,rate,t_ref", [
+    (5, 3, 1, 3, 500.0, 2.0),
+    (161, 150, 1, 1, 3000.0, 0.0),       # lists past the fold's registers
+    (6100, 20, 1, 12, 200.0, 2.0),       # one chunk a warp, piece by piece
+    (6000, 700, 2, 30, 200.0, 2.0),      # more list starts than a warp keeps
+    (12200, 40, 4, 9, 200.0, 2.0),       # two chunks a warp; delays past one step
+    (12400, 150, 1, 254, 100.0, 2.0),    # the grid
+    (30000, 1300, 3, 40, 200.0, 2.0),    # the grid, more list starts than a warp keeps
+    (130001, 30, 1, 16, 60.0, 2.0),      # four neurons a lane
+])
+def test_deterministic(O, n, k, dmin, dmax, rate, t_ref):
+    """Random weights: sums in the canonical order, bit for bit."""
+    s = mixed_net(n, k, dmin, dmax, sources=50, rate=rate, t_ref_ms=t_ref)
+    for c in s.conns[:2]:
+        c.weight, c.wmin, c.wmax = 0.0, 0.05, 0.9
+    assert_matches(O, s.with_(deterministic=True), [1, 64, 40])
+
+
+@pytest.mark.parametrize("n,k", [(900, 60), (14000, 60), (5000, 600)])
+def test_deterministic_plasticity(O, n, k):
+    s = S.plastic_indegree(n=n, k=k, seed=5, drive_rate_hz=60.0).with_(deterministic=True)
+    assert_matches(O, s, [1, 200, 64])
+
+
 @pytest.mark.parametrize("n", [5000, 14000])
 def test_more_spikes_than_the_shared_list(O, n):
     """Every driven neuron fires nearly every step (no refractory period):
