@@ -271,8 +271,8 @@ void throw_device_status(naer::Engine& eng) {
 int naer_net_finish(naer_net* net) {
     return guarded([&] {
         need_compiled(net);
-        net->eng->sync();
-        throw_device_status(*net->eng);
+        throw_device_status(*net->eng);  // waits for the stream
+        NAER_CK(cudaGetLastError());
     });
 }
 
@@ -444,13 +444,11 @@ int naer_net_get_stats(naer_net* net, naer_stats* st) {
     return guarded([&] {
         need_compiled(net);
         need(st != nullptr, NAER_E_INVALID, "null argument");
-        const naer::Ctl c = net->eng->read_ctl();
         std::memset(st, 0, sizeof(*st));
+        const naer::Ctl c = net->eng->read_totals(&st->events, &st->stdp_hist_overflow);
         st->step = c.step;
-        st->events = net->eng->events_total();
         st->spikes = std::min<uint64_t>(c.raster_next, net->net.params.raster_capacity);
         st->raster_dropped = c.raster_dropped;
-        st->stdp_hist_overflow = net->eng->overflow_total();
         st->synapses = net->net.synapses;
         st->device_bytes = net->eng->device_bytes();
         st->neurons = net->net.n_ids;
@@ -496,15 +494,7 @@ namespace {
 void read_state_of(naer::Engine& eng, const naer::NetHost& n, float* v, uint32_t* refractory) {
     std::vector<float> hv(n.n_storage);
     std::vector<uint8_t> hr(n.n_storage);
-    eng.sync();
-    int prev = -1;
-    NAER_CK(cudaGetDevice(&prev));
-    NAER_CK(cudaSetDevice(eng.device()));
-    const cudaError_t e1 = cudaMemcpy(hv.data(), n.v, n.n_storage * 4ull, cudaMemcpyDeviceToHost);
-    const cudaError_t e2 = cudaMemcpy(hr.data(), n.refr, n.n_storage, cudaMemcpyDeviceToHost);
-    cudaSetDevice(prev);
-    NAER_CK(e1);
-    NAER_CK(e2);
+    eng.read_back({{hv.data(), n.v, n.n_storage * 4ull}, {hr.data(), n.refr, n.n_storage}});
     for (const auto& p : n.pops) {
         const bool lif = p.type != naer::kPOISSON;
         for (uint32_t k = 0; k < p.size; ++k) {
@@ -779,13 +769,11 @@ int naer_batch_get_stats(naer_batch* batch, naer_stats* st) {
         naer::Batch& b = *batch->b;
         need(b.compiled(), NAER_E_STATE, "batch is not compiled");
         naer::Engine& eng = b.engine();
-        const naer::Ctl c = eng.read_ctl();
         std::memset(st, 0, sizeof(*st));
+        const naer::Ctl c = eng.read_totals(&st->events, &st->stdp_hist_overflow);
         st->step = c.step;
-        st->events = eng.events_total();
         st->spikes = c.raster_next;
         st->raster_dropped = c.raster_dropped;
-        st->stdp_hist_overflow = eng.overflow_total();
         st->device_bytes = eng.device_bytes();
         for (size_t i = 0; i < b.size(); ++i) {
             st->synapses += b.member((uint32_t)i).synapses;

@@ -2,7 +2,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -183,6 +185,13 @@ public:
     void run_fixed_scratch(uint64_t nsteps);
     void sync();
     Ctl read_ctl();
+    struct ReadBack {
+        void* dst;
+        const void* src;
+        size_t bytes;
+    };
+    // parts of device memory, after the stream's work so far
+    void read_back(std::initializer_list<ReadBack> parts);
     uint64_t host_step() const { return host_step_; }
 
     // raster records [first, first+cap) -> (step, id); returns count copied
@@ -205,7 +214,8 @@ public:
     // launches of this library's own step kernels since creation
     uint64_t kernel_launches() const { return launches_; }
     uint64_t events_total();
-    uint64_t overflow_total();
+    // the control block, with the events delivered and the lazy-LTP overflows so far
+    Ctl read_totals(uint64_t* events, uint64_t* overflow);
 
     void* dalloc(size_t bytes);
     void dfree(void* p, size_t bytes);
@@ -306,6 +316,9 @@ private:
 
 
     uint32_t* h_pinned_ = nullptr;  // small pinned staging
+    static constexpr size_t kReadBackBytes = 64 << 10;
+    static constexpr uint64_t kReadBackRecords = 2048;  // raster records read with their count, at most
+    std::mutex read_back_mu_;       // of its staging
 
     bool failed_ = false;  // a launch reported a device error: state undefined
     void check_usable() const;
