@@ -36,7 +36,7 @@
 // pipes are below 10 % busy.  Per grid step, against k_drive + k_step: 5k
 // neurons / out-degree 100: 3.5 against 9.5 us; 50k / in-degree 400: 5.4
 // against 11.0; 200k / 1000: 11.0 against 12.1; 100k plastic / 1000: 11.9
-// against 12.8; Brunel (delay 15 steps, called window by window) 2k: 1.7
+// against 14.5; Brunel (delay 15 steps, called window by window) 2k: 1.7
 // against 8.6, 60k / 1.8e8 synapses: 7.1 against 17.0.
 namespace naer {
 
@@ -553,6 +553,11 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     const uint32_t rank = kGrid ? blockIdx.x : blockIdx.x % csz, group = kGrid ? 0u : blockIdx.x / csz;
     const bool several = !kGrid && eng.n_nets > 1;
     const bool drawer = wib >= kGroupSteppers;
+    // the grid's drawing warps deliver too once they have drawn, with
+    // plasticity: its items are one synapse a lane, each a chain of loads, and
+    // more warps keep more of them in flight (100k / 1000: 12.6 -> 11.9 us a
+    // step; static rows 14.5 and 14.6, so theirs stay with the others)
+    constexpr bool kDrawersDeliver = kGrid && kPlastic && !kDet;
     const uint32_t nwarps = csz * kGroupSteppers, gw = rank * kGroupSteppers + wib;  // stepping warps
     Ctl* ctl = eng.ctl;
     const uint32_t own_max = eng.group_own;  // neurons of a block, at most
@@ -925,11 +930,13 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                     for (uint32_t at = (wib - kGroupSteppers) * kDrawStep; at < places; at += kGroupDrawers * kDrawStep)
                         qn = group_draw<kPer>(np, sh.pop, s_gc, at, places, d, q, qn, lane, ctl);
                 if (drawn < goal) drawn = goal;
-            } else if (Q) {
+            }
+            if (Q && (!drawer || (kDrawersDeliver && !local))) {
                 // row pieces: enough items for the workers, no more than
                 // the longest row has; one synapse a lane where that
                 // still leaves every worker at most one
-                workers = local ? kGroupSteppers : nwarps;
+                workers = local ? kGroupSteppers : kDrawersDeliver ? csz * kGroupWarps : nwarps;
+                const uint32_t first = local ? wib : drawer ? nwarps + rank * kGroupDrawers + (wib - kGroupSteppers) : gw;
                 const uint32_t narrow = (np.max_row + kPlasticPiece - 1) / kPlasticPiece;
                 const bool stdp = kPlastic && np.stdp_on;
                 wide = (kDet || !stdp) && Q * narrow > workers;
@@ -938,7 +945,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 split = want < pieces ? want : (pieces ? pieces : 1u);
                 items = Q * split;  // at most Q + 2 * workers
                 BinTable bt{};
-                for (uint32_t it = local ? wib : gw; it < items; it += workers) {
+                for (uint32_t it = first; it < items; it += workers) {
                     const uint32_t e = it / split, piece = it - e * split;
                     uint4 head, row;
                     fetch(e, head, row);
