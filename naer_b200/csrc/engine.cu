@@ -849,10 +849,10 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
                 chunks.push_back(ChunkDev{pidx, f, ps.storage_base + ps.size, ni});
         }
         d.pop_count = (uint32_t)pops.size() - d.pop_first;
-        // no spike reaches a neuron in less than the smallest delay
-        d.window = kGroupMaxWindow;
+        uint32_t smallest_delay = kGroupMaxWindow;  // of the connections that have synapses
         for (const ConnSpec& c : n.conns)
-            if (n.pops[c.src].size && n.pops[c.dst].size) d.window = std::min(d.window, c.spec.delay_min);
+            if (n.pops[c.src].size && n.pops[c.dst].size) smallest_delay = std::min(smallest_delay, c.spec.delay_min);
+        d.window = window_steps(smallest_delay, n.ring_slots);
         if (d.stdp_on) d.window = 1;  // a weight update sees the post-synaptic state of its own step
         if (aggregation == NAER_AGG_DETERMINISTIC) d.window = 1;  // events are ordered step by step
         h_nets_.push_back(d);

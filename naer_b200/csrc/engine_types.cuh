@@ -52,6 +52,17 @@ constexpr uint32_t kGroupSeg = 64;        // chunks of a raster segment
 constexpr uint32_t kRasterThreads = 256;
 constexpr uint32_t kGcLif = 1u << 16, kGcDrawn = 1u << 17;  // GroupChunk::info: LIF neurons; Poisson counts are drawn
 
+// Steps of a window of k_group.  No spike may reach a neuron within it: at
+// most the smallest delay.  Its first phase reads and clears one ring slot for
+// each of its steps ahead of the current one: fewer than the ring has (a ring
+// follows from the largest delay declared, so that of a network whose
+// populations are not connected has two slots).
+inline uint32_t window_steps(uint32_t smallest_delay, uint32_t ring_slots) {
+    uint32_t w = smallest_delay < kGroupMaxWindow ? smallest_delay : kGroupMaxWindow;
+    if (w + 1 > ring_slots) w = ring_slots - 1;
+    return w ? w : 1;
+}
+
 struct PopDev {
     uint32_t net;           // owning net slot
     uint32_t type;          // NeuronType
@@ -138,7 +149,7 @@ struct NetDev {
     float fx_scale;
     float fx_inv;
     // k_group
-    uint32_t window;        // steps per window: the smallest delay (1 with plasticity on), <= kGroupMaxWindow
+    uint32_t window;        // steps per window (window_steps; 1 with plasticity on)
     uint32_t pop_first;     // the network's populations: EngineDev::pops [pop_first, pop_first + pop_count)
     uint32_t pop_count;
     uint32_t g_first;       // its chunks: EngineDev::group_chunks [g_first, g_first + g_chunks)
