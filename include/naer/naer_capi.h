@@ -318,14 +318,15 @@ NAER_API int naer_test_fail_allocation(int64_t after);
 /* The bounds-checked build (libnaer_b200_checked.so, compiled with
  * NAER_CHECKED; no counterpart in the reference).  Its step kernels check
  * every global access at a computed index against the buffer it falls in
- * and skip it when outside; the first such index is recorded.  *checked =
- * 1 in that build, 0 in the normal one. */
+ * and skip it when outside; the first such index is recorded, and finish of
+ * a network or batch then fails (NAER_E_CUDA).  *checked = 1 in that build, 0
+ * in the normal one. */
 NAER_API int naer_build_checked(int* checked);
 /* First out-of-bounds access the checked build recorded for the network's
  * launches (*code 0 = none; 1 synapse arrays, 2 ring cell, 3 source of a
  * queued spike, 5 neuron state of a LIF chunk, 6 Poisson-count slot,
- * 8 deterministic event list) and its index.  Always 0 in the normal
- * build.  Blocks like finish(). */
+ * 8 deterministic event list, 9 spike bits of a launch, 10 spike record of a
+ * block) and its index.  Always 0 in the normal build.  Blocks like finish(). */
 NAER_API int naer_net_check_report(naer_net* net, uint32_t* code, uint64_t* index);
 
 /* ---- device probe ------------------------------------------------------

@@ -19,6 +19,8 @@ enum CheckCode : uint32_t {
     kChkState = 5,      // neuron state of a LIF chunk
     kChkDrive = 6,      // Poisson-count slot
     kChkEventList = 8,  // deterministic event list (synapse slot)
+    kChkBits = 9,       // spike bits of a launch (k_group)
+    kChkRecord = 10,    // spike record of a block (k_group)
 };
 
 #ifdef NAER_CHECKED

@@ -1851,6 +1851,11 @@ void Engine::set_barrier_skew(uint64_t skew) {
 
 int Engine::device_status() {
     const Ctl c = read_ctl();  // waits for the stream
+#ifdef NAER_CHECKED
+    if (c.chk_code)
+        throw Error(NAER_E_CUDA, "checked build: out-of-bounds access, code " + std::to_string(c.chk_code) + ", index " +
+                                     std::to_string(c.chk_index));
+#endif
     if (c.error == 0) return 0;
     failed_ = true;
     return c.error == (unsigned int)(-NAER_STATUS_TIMEOUT) ? NAER_E_TIMEOUT : NAER_E_CUDA;

@@ -113,6 +113,15 @@ __device__ __forceinline__ uint4 cluster_ld4(uint32_t a) {
     return v;
 }
 
+// NAER_CHECKED: a ring cell inside the ring, a spike record inside its
+// block's part of the queue.
+__device__ __forceinline__ bool ring_ok(const NetDev& np, uint32_t slot, uint32_t i, Ctl* ctl) {
+    return NAER_IN_BOUNDS(ctl, slot, np.ring_slots, kChkRing) && NAER_IN_BOUNDS(ctl, i, np.n_storage, kChkRing);
+}
+__device__ __forceinline__ bool record_ok(const NetDev& np, uint32_t x, Ctl* ctl) {
+    return NAER_IN_BOUNDS(ctl, x, np.q_cap, kChkRecord);
+}
+
 // Inclusive sum over the warp's lanes.
 __device__ __forceinline__ uint32_t warp_scan(uint32_t x, uint32_t lane) {
 #pragma unroll
@@ -268,7 +277,7 @@ __device__ __forceinline__ void group_row(const NetDev& np, uint32_t slot, float
     const uint8_t* __restrict__ d_a = np.dly + beg;
     uint32_t n = 0;
     auto deliver = [&](uint32_t tgt, float w, uint32_t d) {
-        if (tgt == kTgtSentinel || !NAER_IN_BOUNDS(ctl, tgt, Ns, kChkRing)) return;
+        if (tgt == kTgtSentinel || !ring_ok(np, ring_slot(slot, d, D), tgt, ctl)) return;
         if (mult != 1.0f) w = __fmul_rn(w, mult);
         float* cell = ring + (size_t)ring_slot(slot, d, D) * Ns + tgt;
         if (qs != 0.0f) red_add_s32(cell, __float2int_rn(__fmul_rn(w, qs)));
@@ -301,7 +310,7 @@ __device__ __forceinline__ void group_row(const NetDev& np, uint32_t slot, float
 // g, by one warp.
 __device__ __forceinline__ uint4 raster_bits(const EngineDev& eng, const GroupSeg& seg, uint32_t k, uint32_t x) {
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (x < seg.count) {
+    if (x < seg.count && NAER_IN_BOUNDS(eng.ctl, seg.word + (x + 1) * seg.per - 1, eng.group_words, kChkBits)) {
         const uint32_t* bits = eng.group_bits + (size_t)k * eng.group_words + seg.word;
         if (seg.per == 4) m = __ldcg(reinterpret_cast<const uint4*>(bits) + x);
         else m.x = __ldcg(bits + x);
@@ -458,7 +467,7 @@ __device__ __forceinline__ uint32_t det_link(const NetDev& np, uint32_t tl, uint
         }
 #pragma unroll
         for (uint32_t u = 0; u < (uint32_t)kBatch; ++u) {
-            const bool on = tgt[u] != kTgtSentinel && NAER_IN_BOUNDS(ctl, tgt[u], Ns, kChkRing);
+            const bool on = tgt[u] != kTgtSentinel && ring_ok(np, ring_slot(tmod, d[u], D), tgt[u], ctl);
             cell[u] = on ? ring_slot(tmod, d[u], D) * Ns + tgt[u] : kTgtSentinel;
             if (!on) continue;
             const uint32_t x = off + 32 * u + lane;
@@ -527,7 +536,7 @@ __device__ __forceinline__ void det_refold(const NetDev& np, uint32_t tmod, uint
             const uint32_t tgt = __ldcg(tgt_a + x), d = __ldcg(d_a + x);
             next[u] = __ldcg(np.ev_next + beg + x);
             w[u] = __ldcg(np.ev_w + beg + x);
-            if (tgt != kTgtSentinel && NAER_IN_BOUNDS(ctl, tgt, np.n_storage, kChkRing))
+            if (tgt != kTgtSentinel && ring_ok(np, ring_slot(tmod, d, np.ring_slots), tgt, ctl))
                 cell[u] = ring_slot(tmod, d, np.ring_slots) * np.n_storage + tgt;
         }
 #pragma unroll
@@ -666,6 +675,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 eng.record ? eng.group_bits + (size_t)(s - s0) * eng.group_words + np.g_word : nullptr;
             // spikes of one step of a chunk as bits for the raster
             auto put_bits = [&](uint32_t hit, uint32_t k, uint32_t chunk) {
+                if (!NAER_IN_BOUNDS(ctl, s - s0 + k, nsteps, kChkBits) ||
+                    !NAER_IN_BOUNDS(ctl, np.g_word + (chunk + 1) * kPer - 1, eng.group_words, kChkBits))
+                    return;
                 uint32_t* to = bits + (size_t)k * eng.group_words + chunk * kPer;
                 if constexpr (kPer == 4) {
                     uint32_t m[4];
@@ -687,6 +699,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                 pos = __shfl_sync(0xFFFFFFFFu, pos, 31) + x - n;
                 for (; hits; hits &= hits - 1, ++pos) {
                     const uint32_t bit = __ffsll(hits) - 1, k = bit / kPer, u = bit % kPer;
+                    if (!NAER_IN_BOUNDS(ctl, i + u, Ns, kChkState) || !record_ok(np, pos, ctl)) continue;
                     // a POISSON source's multiplicity is its count
                     const uint32_t m = lif ? 0u : __ldcg(np.drive + (size_t)((s + k) % kDriveSlots) * Ns + i + u);
                     const uint4 row = eng.group_rows ? s_row[at + u] : row_of(np.row_ptr, np.row_mid, i + u);
@@ -751,7 +764,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                     for (uint32_t u = 0; u < kTile; ++u) {
                         if (u && j0 + u >= own) break;
                         gc[u] = s_gc[(j0 + u) * kGroupSteppers + wib];
-                        const bool on = kPer * lane < ((gc[u].y >> 8) & 0xFFu);
+                        const bool on = kPer * lane < ((gc[u].y >> 8) & 0xFFu) &&
+                                        ring_ok(np, tmod, gc[u].x + kPer * lane + kPer - 1, ctl);
                         dr[u] = on && (gc[u].y & kGcDrawn) ? ld_bytes<kPer>(drive + gc[u].x) : 0u;
                         if (on && (gc[u].y & kGcLif)) {
                             in[u] = ld_vals<kPer>(ring + gc[u].x);
@@ -768,7 +782,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         const bool lif = gc[u].y & kGcLif;
                         uint32_t hit = 0;
                         if (lif) {
-                            if (kPer * lane < count) {
+                            if (kPer * lane < count && ring_ok(np, tmod, gc[u].x + kPer * lane + kPer - 1, ctl)) {
                                 clear_vals<kPer>(ring + gc[u].x);
                                 const PopDev& p = sh.pop[gc[u].y & 0xFFu];
                                 const GroupLif prm{p.prop, p.v_th, p.v_reset, p.drive_w, fx_inv, p.t_ref_steps};
@@ -792,7 +806,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                     const uint2 gc = s_gc[j * kGroupSteppers + wib];
                     const uint32_t i = gc.x + kPer * lane, at = (j * kGroupSteppers + wib) * kChunk + kPer * lane;
                     const uint32_t valid = valid_of((gc.y >> 8) & 0xFFu);
-                    const bool on = valid != 0, lif = gc.y & kGcLif, drawn_pop = gc.y & kGcDrawn;
+                    const bool on = valid != 0 && NAER_IN_BOUNDS(ctl, i + kPer - 1, Ns, kChkState);
+                    const bool lif = gc.y & kGcLif, drawn_pop = gc.y & kGcDrawn;
                     const PopDev& p = sh.pop[gc.y & 0xFFu];
                     const GroupLif prm{p.prop, p.v_th, p.v_reset, p.drive_w, fx_inv, p.t_ref_steps};
                     Vals<kPer> v;
@@ -806,7 +821,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         uint32_t dr[kStepTile];
 #pragma unroll
                         for (uint32_t u = 0; u < kStepTile; ++u) {
-                            const bool step_on = on && k0 + u < w;
+                            const bool step_on =
+                                on && k0 + u < w && ring_ok(np, ring_slot(tmod, k0 + u, D), i + kPer - 1, ctl);
                             dr[u] = step_on && drawn_pop
                                         ? ld_bytes<kPer>(np.drive + (size_t)((s + k0 + u) % kDriveSlots) * Ns + i)
                                         : 0u;
@@ -820,7 +836,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         if (lif && on) {
 #pragma unroll
                             for (uint32_t u = 0; u < kStepTile; ++u)
-                                if (k0 + u < w) clear_vals<kPer>(np.ring + (size_t)ring_slot(tmod, k0 + u, D) * Ns + i);
+                                if (k0 + u < w && ring_ok(np, ring_slot(tmod, k0 + u, D), i + kPer - 1, ctl))
+                                    clear_vals<kPer>(np.ring + (size_t)ring_slot(tmod, k0 + u, D) * Ns + i);
                         }
 #pragma unroll
                         for (uint32_t u = 0; u < kStepTile; ++u) {
@@ -843,7 +860,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             if (!local) {
                 if (kGrid && threadIdx.x == 0) __stcg(eng.group_cnt + rank, mine);
                 if (!drawer && (kGrid || (kPlastic && np.stdp_on))) {
-                    for (uint32_t e = threadIdx.x; e < mine; e += kGroupStepThreads) {
+                    for (uint32_t e = threadIdx.x; e < mine && record_ok(np, e, ctl); e += kGroupStepThreads) {
                         int4 head;
                         if (e < kGroupList) head = *reinterpret_cast<const int4*>(s_list + e);
                         else head = __ldcg(reinterpret_cast<const int4*>(eng.queue[0] + region + e));
@@ -910,7 +927,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         x = e - sh.first[reg];
                     }
                 }
-                if (local && x < kGroupList) {
+                if (!record_ok(np, x, ctl)) {
+                    head = row = make_uint4(kTgtSentinel, 0u, 0u, 0u);  // no source: skipped by the caller
+                } else if (local && x < kGroupList) {
                     head = *reinterpret_cast<const uint4*>(s_list + x);
                     row = s_list[x].row;
                 } else if (!kGrid && x < kGroupList) {
@@ -979,6 +998,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
                         const uint32_t e = it / split;
                         uint4 head, row;
                         fetch(e, head, row);
+                        if (!NAER_IN_BOUNDS(ctl, head.x, Ns, kChkQueue)) continue;
                         const uint64_t beg = ((uint64_t)row.y << 32) | row.x;
                         if (wide) det_refold<4>(np, tmod, beg, row.w, it - e * split, split, lane, ctl);
                         else det_refold<1>(np, tmod, beg, row.w, it - e * split, split, lane, ctl);
@@ -1003,7 +1023,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const uint32_t place = j * kGroupSteppers + wib;
             const uint2 gc = s_gc[place];
             const uint32_t at = place * kChunk + kPer * lane, i = gc.x + kPer * lane;
-            if (kPer * lane < ((gc.y >> 8) & 0xFFu) && (gc.y & kGcLif)) {
+            if (kPer * lane < ((gc.y >> 8) & 0xFFu) && (gc.y & kGcLif) &&
+                NAER_IN_BOUNDS(ctl, i + kPer - 1, np.n_storage, kChkState)) {
                 if constexpr (kPer == 4) {
                     *reinterpret_cast<float4*>(np.v + i) = *reinterpret_cast<const float4*>(sV + at);
                     *reinterpret_cast<uint32_t*>(np.refr + i) = *reinterpret_cast<const uint32_t*>(sR + at);
