@@ -1133,10 +1133,8 @@ bool Engine::plan_one(const std::vector<PopDev>& pops) {
     k.own = group_own(d, pops, c, k.per);
     k.stdp = d.stdp_on != 0;
     k.det = det;
-    // the windows' spike records (32 B each) stay below 256 MB
-    const uint64_t most_entries = 8000000;
-    if (!cluster && (uint64_t)c * k.own * d.window > most_entries)
-        d.window = (uint32_t)std::max<uint64_t>(1, most_entries / ((uint64_t)c * k.own));
+    if (!cluster && (uint64_t)c * k.own * d.window > kGroupMostRecords)
+        d.window = (uint32_t)std::max<uint64_t>(1, kGroupMostRecords / ((uint64_t)c * k.own));
     if (!cluster && d.window == 1 && n.n_storage > (det ? d.stdp_on ? 600000u : 250000u : d.stdp_on ? 250000u : 500000u))
         return false;
     if (!fit_class(k)) return false;
@@ -1260,6 +1258,18 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
             if (!fit_class(c)) return false;
             group_classes_.push_back(c);
         }
+    // the longest windows shortened to what the records allow
+    uint32_t longest = kGroupMaxWindow;
+    for (; longest > 1; --longest) {
+        uint64_t records = 0;
+        for (size_t i = 0; i < count; ++i) {
+            const uint32_t c = sizes[best_pick[i]];
+            records += (uint64_t)group_own(h_nets_[i], pops, c, per_of(h_nets_[i], c)) * c *
+                       std::min(longest, h_nets_[i].window);
+        }
+        if (records <= kGroupMostRecords) break;
+    }
+    for (NetDev& d : h_nets_) d.window = std::min(d.window, longest);
     return true;
 }
 

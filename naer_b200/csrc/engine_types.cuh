@@ -49,6 +49,8 @@ constexpr uint32_t kGroupMaxBlocks = 160; // blocks of a group, at most
 constexpr uint32_t kGroupPops = 8;        // populations of a network, at most
 constexpr uint32_t kGroupList = 1024;     // spikes of a window a block keeps in shared memory
 constexpr uint32_t kGroupSeg = 64;        // chunks of a raster segment
+// spike records (32 B each) of all blocks, at most, where windows are longer than one step
+constexpr uint64_t kGroupMostRecords = 8000000;
 constexpr uint32_t kRasterThreads = 256;
 constexpr uint32_t kGcLif = 1u << 16, kGcDrawn = 1u << 17;  // GroupChunk::info: LIF neurons; Poisson counts are drawn
 
