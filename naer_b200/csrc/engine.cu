@@ -877,16 +877,7 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     upload(reinterpret_cast<void*&>(d_pops_), pops_bytes_, pops.data(), pops.size() * sizeof(PopDev));
     upload(reinterpret_cast<void*&>(d_chunks_), chunks_bytes_, chunks.data(), chunks.size() * sizeof(ChunkDev));
 
-    if (group_form_ != kGroupNone) {
-        upload(reinterpret_cast<void*&>(d_gchunks_), gchunks_bytes_, h_chunks_.data(), h_chunks_.size() * sizeof(GroupChunk));
-        if (h_nets_.size() > 1)
-            upload(reinterpret_cast<void*&>(d_gorder_), gorder_bytes_, h_order_.data(), h_order_.size() * 4ull);
-        upload(reinterpret_cast<void*&>(d_gsegs_), gsegs_bytes_, h_segs_.data(), h_segs_.size() * sizeof(GroupSeg));
-    }
-
-    const EngineDev planned = eng_;
     eng_ = EngineDev{};
-    eng_.group_words = planned.group_words;
     eng_.n_chunks = (uint32_t)chunks.size();
     eng_.n_nets = (uint32_t)nets.size();
 
@@ -953,13 +944,10 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     // k_det_step)
     const uint64_t qentries = list_kernel ? std::max<uint64_t>(qcap, 1) : std::max<uint64_t>((uint64_t)lif_grid_ * region_cap, qcap);
     if (qentries > 0xFFFFFFFFull) throw Error(NAER_E_OVERFLOW, "spike queue larger than 2^32 entries");
-    const uint64_t gentries = group_form_ != kGroupNone ? group_entries_ : 0;
     for (int i = 0; i < 2; ++i) {
-        regrow(reinterpret_cast<void*&>(d_queue_[i]), queue_bytes_[i],
-               std::max(qentries, i == 0 ? gentries : 0) * sizeof(SpikeRec));
+        regrow(reinterpret_cast<void*&>(d_queue_[i]), queue_bytes_[i], qentries * sizeof(SpikeRec));
         regrow(reinterpret_cast<void*&>(d_qid_[i]), qid_bytes_[i], qentries * sizeof(uint32_t));
-        regrow(reinterpret_cast<void*&>(d_qrow_[i]), qrow_bytes_[i],
-               std::max(qentries, i == 0 ? gentries : 0) * sizeof(uint4));
+        regrow(reinterpret_cast<void*&>(d_qrow_[i]), qrow_bytes_[i], qentries * sizeof(uint4));
         regrow(reinterpret_cast<void*&>(d_counts_[i]), counts_bytes_[i], (lif_grid_ + 1) * sizeof(uint32_t));
         NAER_CK(cudaMemsetAsync(d_counts_[i], 0, (lif_grid_ + 1) * sizeof(uint32_t), stream_));
     }
@@ -991,23 +979,6 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     }
     eng_.ev_part = d_ev_part_;
     eng_.ovf_part = d_ovf_part_;
-    if (group_form_ != kGroupNone) {
-        const uint64_t steps = group_launch_steps();
-        regrow(reinterpret_cast<void*&>(d_gcnt_), gcnt_bytes_, group_blocks_ * 4ull);
-        NAER_CK(cudaMemsetAsync(&d_ctl_->raster_done, 0, 4, stream_));
-        if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * eng_.group_words * 4ull);
-        regrow(reinterpret_cast<void*&>(d_gq_), gq_bytes_, steps * h_segs_.size() * 4ull);
-        NAER_CK(cudaMemsetAsync(d_gq_, 0, steps * h_segs_.size() * 4ull, stream_));
-        regrow(reinterpret_cast<void*&>(d_gtot_), gtot_bytes_, steps * 4ull);
-        NAER_CK(cudaMemsetAsync(d_gtot_, 0, steps * 4ull, stream_));
-        eng_.group_segs = d_gsegs_;
-        eng_.group_seg_n = (uint32_t)h_segs_.size();
-        eng_.group_tot = d_gtot_;
-        eng_.group_chunks = d_gchunks_;
-        eng_.group_cnt = d_gcnt_;
-        eng_.group_bits = d_gbits_;
-        eng_.group_q = d_gq_;
-    }
     eng_.raster = d_raster_;
     eng_.raster_cap = raster_capacity;
     eng_.lif_grid = lif_grid_;
@@ -1045,7 +1016,61 @@ void Engine::install(const std::vector<NetHost*>& nets, uint64_t raster_capacity
     eng_.bins = bins;
     if (qentries * std::max(eng_.split_first, eng_.split_rest) > 0xFFFFFFFFull)
         throw Error(NAER_E_OVERFLOW, "spike list times warps per spike exceeds 2^32 work items");
+    // k_group's own tables and buffers last: without memory for them the
+    // networks step on the grid kernels, for which everything is in place
+    if (group_form_ != kGroupNone) {
+        try {
+            upload(reinterpret_cast<void*&>(d_gchunks_), gchunks_bytes_, h_chunks_.data(), h_chunks_.size() * sizeof(GroupChunk));
+            if (h_nets_.size() > 1)
+                upload(reinterpret_cast<void*&>(d_gorder_), gorder_bytes_, h_order_.data(), h_order_.size() * 4ull);
+            upload(reinterpret_cast<void*&>(d_gsegs_), gsegs_bytes_, h_segs_.data(), h_segs_.size() * sizeof(GroupSeg));
+            const uint64_t steps = group_launch_steps();
+            regrow(reinterpret_cast<void*&>(d_gcnt_), gcnt_bytes_, group_blocks_ * 4ull);
+            NAER_CK(cudaMemsetAsync(&d_ctl_->raster_done, 0, 4, stream_));
+            if (record) regrow(reinterpret_cast<void*&>(d_gbits_), gbits_bytes_, steps * group_words_ * 4ull);
+            regrow(reinterpret_cast<void*&>(d_gq_), gq_bytes_, steps * h_segs_.size() * 4ull);
+            NAER_CK(cudaMemsetAsync(d_gq_, 0, steps * h_segs_.size() * 4ull, stream_));
+            regrow(reinterpret_cast<void*&>(d_gtot_), gtot_bytes_, steps * 4ull);
+            NAER_CK(cudaMemsetAsync(d_gtot_, 0, steps * 4ull, stream_));
+            // the blocks' spike records
+            regrow(reinterpret_cast<void*&>(d_queue_[0]), queue_bytes_[0], group_entries_ * sizeof(SpikeRec));
+            regrow(reinterpret_cast<void*&>(d_qrow_[0]), qrow_bytes_[0], group_entries_ * sizeof(uint4));
+        } catch (const Error& e) {
+            if (e.code != NAER_E_OOM) throw;
+            group_form_ = kGroupNone;
+            free_group();
+            regrow(reinterpret_cast<void*&>(d_queue_[0]), queue_bytes_[0], qentries * sizeof(SpikeRec));
+            regrow(reinterpret_cast<void*&>(d_qrow_[0]), qrow_bytes_[0], qentries * sizeof(uint4));
+        }
+        eng_.queue[0] = d_queue_[0];
+        eng_.qrow[0] = d_qrow_[0];
+    }
+    if (group_form_ != kGroupNone) {
+        eng_.group_words = group_words_;
+        eng_.group_segs = d_gsegs_;
+        eng_.group_seg_n = (uint32_t)h_segs_.size();
+        eng_.group_tot = d_gtot_;
+        eng_.group_chunks = d_gchunks_;
+        eng_.group_cnt = d_gcnt_;
+        eng_.group_bits = d_gbits_;
+        eng_.group_q = d_gq_;
+    }
     NAER_CK(cudaStreamSynchronize(stream_));  // tables and buffers complete for every stream
+}
+
+void Engine::free_group() {
+    auto f = [&](auto*& p, size_t& bytes) {
+        if (p) dfree(p, bytes);
+        p = nullptr;
+        bytes = 0;
+    };
+    f(d_gchunks_, gchunks_bytes_);
+    f(d_gorder_, gorder_bytes_);
+    f(d_gsegs_, gsegs_bytes_);
+    f(d_gcnt_, gcnt_bytes_);
+    f(d_gbits_, gbits_bytes_);
+    f(d_gq_, gq_bytes_);
+    f(d_gtot_, gtot_bytes_);
 }
 
 // 32 x per neurons of one population a warp takes at a time.
@@ -1321,7 +1346,7 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
             d.q_off = group_entries_;
             group_entries_ += (uint64_t)d.q_cap * c.size;
         }
-        eng_.group_words = (words + 3u) & ~3u;
+        group_words_ = (words + 3u) & ~3u;
     }
     if (ok && group_entries_ > 1000000) {  // not where the device is nearly full
         size_t free_b = 0, total_b = 0;

@@ -258,6 +258,7 @@ private:
     const void* group_kernel(const GroupClass& c) const;
     bool group_active() const { return group_form_ == kGroupGrid || (group_form_ == kGroupCluster && bar_skew_ == 0); }
     void launch_group(uint32_t steps, bool from_ctl);
+    void free_group();
     uint32_t group_launch_steps() const { return tuning_.group_steps ? tuning_.group_steps : tuning_.launch_steps; }
     void launch_run(uint32_t steps);
     void launch_drive(uint64_t s_first, uint32_t nsteps);
@@ -347,6 +348,7 @@ private:
     uint32_t* d_gbits_ = nullptr;
     uint32_t* d_gq_ = nullptr;
     size_t gchunks_bytes_ = 0, gcnt_bytes_ = 0, gbits_bytes_ = 0, gq_bytes_ = 0;
+    uint32_t group_words_ = 0;  // words of spike bits of one step
     // CUDA-event timing of launches while profiling (pairs in launch order)
     std::vector<cudaEvent_t> timer_events_;
     std::vector<int> timer_kinds_;  // 0 drive, 1 step kernel

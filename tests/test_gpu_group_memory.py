@@ -1,12 +1,14 @@
 """Device memory of the window kernel: the spike records of a batch's windows
-are bounded."""
+are bounded, and without memory for its buffers a network steps on the grid
+kernels instead of failing to compile."""
 import numpy as np
 import pytest
 
+from naer_b200 import _capi as capi
+from naer_b200 import spec as S
 from naer_b200.forms import Batch
 
 from test_gpu_group import mixed_net
-from naer_b200 import spec as S
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +34,41 @@ def test_records_of_long_windows_are_bounded(lib):
             net.finish()
             want = net.read_spikes() + net.read_state()
         assert len(want[1]) > 100 and all(np.array_equal(x, y) for x, y in zip(g, want))
+
+
+def test_no_memory_for_its_buffers(lib):
+    """Every allocation of a compile fails in turn: one of the window kernel's
+    own leaves the network compiled, on k_drive + k_step (two launches of up to
+    64 steps), with the same results and no more memory than those need."""
+    s = mixed_net(14_000, 12, 12, 14, sources=33)
+    with S.build(s) as net:
+        net.run(64)
+        net.finish()
+        want = net.read_spikes() + net.read_state()
+        assert net.stats()["kernel_launches"] == 1
+        most = net.stats()["device_bytes"]
+    fell_back = 0
+    try:
+        for k in range(400):
+            net = S.describe(s, device=0)
+            try:
+                capi.call("naer_test_fail_allocation", k)
+                rc = lib.naer_net_compile(net.handle)
+                capi.call("naer_test_fail_allocation", -1)
+                if rc == capi.NAER_E_OOM:
+                    continue
+                assert rc == capi.NAER_OK
+                net.run(64)
+                net.finish()
+                launches = net.stats()["kernel_launches"]
+                got = net.read_spikes() + net.read_state()
+                assert all(np.array_equal(x, y) for x, y in zip(got, want)), k
+                if launches == 1:
+                    break  # no allocation failed
+                assert launches == 2 and net.stats()["device_bytes"] < most, k
+                fell_back += 1
+            finally:
+                net.close()
+    finally:
+        capi.call("naer_test_fail_allocation", -1)
+    assert launches == 1 and fell_back >= 6  # chunks, segments, counts, spike bits, records
