@@ -393,7 +393,12 @@ typedef struct naer_tuning {
  * while the grid waits at its barriers.  TWO_BARRIER: per-block spike
  * regions, the whole scatter between two grid barriers.  Same results; both
  * serve atomic and exact-sum aggregation (deterministic aggregation has a
- * kernel of its own). */
+ * kernel of its own).
+ * SPLIT is also the default, and with it and no geometry of its own
+ * (blocks_per_sm, scatter_split, scatter_piece, neuron_state and bins all 0)
+ * networks step on the window kernel instead where it is expected to be
+ * faster; a geometry, blocks_per_sm = 2 for instance, keeps them on the split
+ * kernel.  The same holds for deterministic aggregation and its kernel. */
 #define NAER_KERNEL_SPLIT 0u
 #define NAER_KERNEL_TWO_BARRIER 1u
 
@@ -466,11 +471,14 @@ typedef struct naer_server_params {
     uint32_t max_jobs;         /* jobs stepped together, at most */
     uint32_t blocks_per_sm;    /* step-kernel blocks per SM (0 = most that fit) */
     double chunk_ms;           /* target device time of a chunk: fewer steps when many jobs run */
-    uint32_t launch_steps;     /* grid steps per persistent step launch, 1..64 (0 = default);
-                                  builds run between launches, so short launches let jobs in sooner
-                                  and long ones pay less launch overhead per step */
-    uint32_t step_kernel;      /* atomic and exact-sum aggregation: NAER_KERNEL_TWO_BARRIER (default; the
-                                  served job mix completes more jobs per second with it) or NAER_KERNEL_SPLIT */
+    uint32_t launch_steps;     /* grid steps per step launch, 1..64 (0 = default: 4 where the jobs step on
+                                  the whole grid, 32 in clusters); builds run between launches, and beside
+                                  clusters, so short launches let jobs in sooner and long ones pay less
+                                  launch overhead per step */
+    uint32_t step_kernel;      /* atomic and exact-sum aggregation: NAER_KERNEL_TWO_BARRIER (default): sets of
+                                  jobs for which it is expected to be faster step in clusters of their own,
+                                  a lone job as a single network does, the others on the two-barrier kernel;
+                                  NAER_KERNEL_SPLIT: every set on the split kernel */
 } naer_server_params;
 
 #define NAER_JOB_QUEUED 0u

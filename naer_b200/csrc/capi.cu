@@ -831,7 +831,7 @@ int naer_server_create(int device, const naer_server_params* params, naer_server
         sp.max_jobs = p.max_jobs;
         sp.blocks_per_sm = p.blocks_per_sm;
         sp.chunk_ms = p.chunk_ms;
-        if (p.launch_steps) sp.launch_steps = p.launch_steps;
+        sp.launch_steps = p.launch_steps;
         need(p.step_kernel <= NAER_KERNEL_TWO_BARRIER, NAER_E_INVALID, "unknown step kernel");
         sp.step_kernel = p.step_kernel;
         auto h = std::make_unique<naer_server>();

@@ -1304,7 +1304,7 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
     group_form_ = kGroupNone;
     group_entries_ = 0;
     const bool det = aggregation_ == NAER_AGG_DETERMINISTIC;
-    if ((det && h_nets_.size() > 1) || !tuning_.group_allowed() || h_nets_.empty()) return;
+    if ((det && h_nets_.size() > 1) || !tuning_.group_allowed(det) || h_nets_.empty()) return;
     bool ok = true;
     for (const NetDev& d : h_nets_) ok = ok && d.pop_count > 0 && d.pop_count <= kGroupPops;
     ok = ok && (h_nets_.size() == 1 ? plan_one(pops) : plan_several(pops));

@@ -122,14 +122,17 @@ struct Tuning {
     uint32_t neuron_state = 0;             // NAER_STATE_AUTO / _SHARED / _GLOBAL: where the step kernel keeps V
     uint32_t step_kernel = 0;              // NAER_KERNEL_SPLIT (k_step) / NAER_KERNEL_TWO_BARRIER (k_run)
     uint32_t bins = 0;                     // k_step shared-memory binning table entries (0 = off)
-    uint32_t group_steps = 0;              // served form: k_group may run whatever step_kernel says, with this
-                                           // many steps per launch (0: as launch_steps)
+    uint32_t group_steps = 0;              // grid steps per launch of clusters (0: as launch_steps)
+    uint32_t group_kernel = 0;             // the step_kernel that leaves k_group open (deterministic aggregation
+                                           // has one kernel besides it: there either does)
 
     // the choices that name a kernel or a geometry of its own are all open
-    bool group_allowed() const {
+    bool group_allowed(bool det) const {
         return blocks_per_sm == 0 && scatter_split == 0 && scatter_piece == 0 && neuron_state == 0 && bins == 0 &&
-               (step_kernel == 0 || group_steps);
+               (step_kernel == group_kernel || (det && group_kernel));
     }
+    // grid steps per launch of k_group, in clusters or on the whole grid
+    uint32_t group_launch_steps(bool clusters) const { return clusters && group_steps ? group_steps : launch_steps; }
 };
 
 struct TuneResult {
@@ -259,7 +262,7 @@ private:
     bool group_active() const { return group_form_ == kGroupGrid || (group_form_ == kGroupCluster && bar_skew_ == 0); }
     void launch_group(uint32_t steps, bool from_ctl);
     void free_group();
-    uint32_t group_launch_steps() const { return tuning_.group_steps ? tuning_.group_steps : tuning_.launch_steps; }
+    uint32_t group_launch_steps() const { return tuning_.group_launch_steps(group_form_ == kGroupCluster); }
     void launch_run(uint32_t steps);
     void launch_drive(uint64_t s_first, uint32_t nsteps);
     void run_launches(uint64_t nsteps);

@@ -99,8 +99,7 @@ Server::Server(int device, const ServerParams& p) : device_(device), prm_(p), t0
     if (p.chunk_steps == 0) throw Error(NAER_E_INVALID, "chunk_steps must be positive");
     if (p.max_jobs == 0) throw Error(NAER_E_INVALID, "max_jobs must be positive");
     if (p.raster_capacity == 0) throw Error(NAER_E_INVALID, "raster_capacity must be positive");
-    if (p.launch_steps == 0 || p.launch_steps > kDriveSlots)
-        throw Error(NAER_E_INVALID, "launch_steps must be in 1..64");
+    if (p.launch_steps > kDriveSlots) throw Error(NAER_E_INVALID, "launch_steps must be in 1..64 (0: default)");
     int n = 0;
     NAER_CK(cudaGetDeviceCount(&n));
     if (device < 0 || device >= n) throw Error(NAER_E_INVALID, "device index out of range");
@@ -404,16 +403,7 @@ void Server::loop() {
         eng = std::make_unique<Engine>(device_);
         // short persistent launches: the builder's kernels (higher-priority
         // stream) get the device between them instead of after whole chunks
-        Tuning tn;
-        tn.launch_steps = prm_.launch_steps;
-        tn.blocks_per_sm = prm_.blocks_per_sm;
-        tn.step_kernel = prm_.step_kernel;
-        // jobs in clusters of their own leave the builder SMs to run on, and a
-        // launch costs as much as two or three steps (24 jobs of up to 20k
-        // neurons, all at once, ms until the last: 35.0 with 16 steps a launch,
-        // 33.8 with 32, 33.0 with 64; 78.6 on the two-barrier kernel)
-        tn.group_steps = std::max<uint32_t>(32, prm_.launch_steps);
-        eng->set_tuning(tn);
+        eng->set_tuning(served_tuning(prm_));
         // Admission keeps the running set within the step kernel's fastest
         // geometry (neuron state in shared memory, most blocks per SM).  A
         // larger set steps more slowly per job, so a backlog that admitted

@@ -54,9 +54,25 @@ struct ServerParams {
     uint64_t raster_capacity = 1ull << 24;  // spike records per chunk
     uint32_t blocks_per_sm = 0;    // step-kernel blocks per SM (0 = most that fit)
     double chunk_ms = 10.0;        // target device time per chunk (sets its step count)
-    uint32_t launch_steps = 4;     // grid steps per persistent step launch (builds run between launches)
-    uint32_t step_kernel = 1;      // NAER_KERNEL_TWO_BARRIER (k_run) / NAER_KERNEL_SPLIT (k_step)
+    uint32_t launch_steps = 0;     // grid steps per step launch (0: served_tuning's)
+    uint32_t step_kernel = 1;      // NAER_KERNEL_TWO_BARRIER: clusters where they pay, else k_run; NAER_KERNEL_SPLIT: k_step
 };
+
+// Launches of the served form.  On the grid kernels and the grid form of
+// k_group builds run between launches: 4 steps.  Jobs in clusters of their own
+// leave the builder SMs to run on, and a launch costs as much as two or three
+// steps: 32 (24 jobs of up to 20k neurons, all at once, ms until the last:
+// 35.0 with 16 steps a launch, 33.8 with 32, 33.0 with 64; 78.6 on the
+// two-barrier kernel).
+inline Tuning served_tuning(const ServerParams& p) {
+    Tuning t;
+    t.launch_steps = p.launch_steps ? p.launch_steps : 4;
+    t.group_steps = p.launch_steps ? p.launch_steps : 32;
+    t.blocks_per_sm = p.blocks_per_sm;
+    t.step_kernel = p.step_kernel;
+    t.group_kernel = NAER_KERNEL_TWO_BARRIER;
+    return t;
+}
 
 enum JobState : uint32_t { kJobQueued = 0, kJobRunning = 1, kJobDone = 2, kJobFailed = 3, kJobCancelled = 4 };
 
