@@ -140,7 +140,8 @@ typedef struct naer_stats {
     uint64_t device_bytes;      /* device memory held by the handle */
     uint32_t neurons;
     uint32_t ring_slots;
-    uint64_t kernel_launches;   /* launches of the library's own step kernels */
+    uint64_t kernel_launches;   /* launches of the library's own step kernels (the clusters of several sizes
+                                   that step a batch beside one another count as one) */
 } naer_stats;
 
 typedef struct naer_net naer_net;
@@ -434,7 +435,9 @@ NAER_API int naer_batch_clear_spikes(naer_batch* batch);
 /* Whole-batch counters (synapses and neurons summed over members). */
 NAER_API int naer_batch_get_stats(naer_batch* batch, naer_stats* st);
 /* The step kernel's phase split for the whole batch, as naer_net_get_phases
- * (ms, accumulated since compile, measured by the kernel's first block). */
+ * (ms, accumulated since compile, measured by the kernel's first block; where
+ * the members step in clusters of their own, the mean over the members of the
+ * times of each one's first block). */
 NAER_API int naer_batch_get_phases(naer_batch* batch, double* phase_ms5);
 NAER_API int naer_batch_read_state(naer_batch* batch, uint32_t member, float* v, uint32_t* refractory);
 NAER_API int naer_batch_stream(naer_batch* batch, void** stream);

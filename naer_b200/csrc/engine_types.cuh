@@ -191,7 +191,8 @@ struct SpikeRec {
 //   raster_next raster records kept so far
 //   bar_arrive  grid barrier arrivals of the persistent kernel (zeroed per launch)
 //   error       first device-side error (negated NAER status), 0 = none
-//   prof_*      phase times of the persistent kernel (block 0, %globaltimer)
+//   prof_*      phase times of the persistent kernel (block 0, of several networks in clusters the mean
+//               of their first blocks; %globaltimer)
 struct Ctl {
     unsigned long long step;
     unsigned long long raster_base;

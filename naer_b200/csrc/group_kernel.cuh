@@ -68,7 +68,7 @@ struct GroupShared {
     uint32_t ovf;
     uint32_t n_spikes[2];                 // spikes of the block in this window, by window parity
     uint32_t first[kGroupMaxBlocks + 1];  // grid form: spikes of the blocks before each
-    unsigned long long ph[4];             // thread 0 of block 0
+    unsigned long long ph[4];             // thread 0 of the group's first block
 };
 
 // Barrier of the group.
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     uint32_t ovf = 0;
     if (s0 == kStepFromCtl) s0 = ctl->step;
     const unsigned long long rbase = ctl->raster_next;
-    const bool timer = blockIdx.x == 0 && eng.group_part == 0 && threadIdx.x == 0;
+    const bool timer = rank == 0 && threadIdx.x == 0;
     if (threadIdx.x == 0) {
         sh.bcfg = barrier_cfg(ctl);
         sh.ok = 1;
@@ -1053,14 +1053,17 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         if (ok && rank == 0) raster_end(eng, s0, nsteps, rbase);
     }
     finish_counters(eng, ev, ovf, lane, &sh.ev, &sh.ovf, eng.group_part);
-    if (timer) {
-        ctl->prof_phase_ns[0] += sh.ph[0];
-        ctl->prof_phase_ns[1] += sh.ph[1];
-        ctl->prof_phase_ns[2] += sh.ph[2];
-        ctl->prof_phase_ns[4] += sh.ph[3];
-        ctl->prof_lif_ns += sh.ph[0] + sh.ph[1];
-        ctl->prof_scatter_ns += sh.ph[2] + sh.ph[3];
-        ctl->prof_steps += nsteps;
+    if (timer) {  // phase times: mean over the networks
+        unsigned long long ph[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) ph[x] = several ? sh.ph[x] / eng.n_nets : sh.ph[x];
+        atomicAdd(&ctl->prof_phase_ns[0], ph[0]);
+        atomicAdd(&ctl->prof_phase_ns[1], ph[1]);
+        atomicAdd(&ctl->prof_phase_ns[2], ph[2]);
+        atomicAdd(&ctl->prof_phase_ns[4], ph[3]);
+        atomicAdd(&ctl->prof_lif_ns, ph[0] + ph[1]);
+        atomicAdd(&ctl->prof_scatter_ns, ph[2] + ph[3]);
+        if (blockIdx.x == 0 && eng.group_part == 0) ctl->prof_steps += nsteps;
     }
 }
 
