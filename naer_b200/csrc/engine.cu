@@ -1370,7 +1370,8 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
 
 template <bool kGrid, int kPer>
 static const void* group_kernel_of(bool stdp, bool det) {
-    if (det) return stdp ? (const void*)k_group<kGrid, kPer, true, true> : (const void*)k_group<kGrid, kPer, false, true>;
+    if constexpr (kGrid || kPer == 1)
+        if (det) return stdp ? (const void*)k_group<kGrid, kPer, true, true> : (const void*)k_group<kGrid, kPer, false, true>;
     return stdp ? (const void*)k_group<kGrid, kPer, true, false> : (const void*)k_group<kGrid, kPer, false, false>;
 }
 const void* Engine::group_kernel(const GroupClass& c) const {

@@ -1090,15 +1090,17 @@ __global__ void __launch_bounds__(kRasterThreads) k_raster(EngineDev eng, unsign
 }
 
 
-#define NAER_GROUP(grid, per)                                                                      \
-    template __global__ void k_group<grid, per, true, false>(EngineDev, unsigned long long, uint32_t);  \
-    template __global__ void k_group<grid, per, false, false>(EngineDev, unsigned long long, uint32_t); \
-    template __global__ void k_group<grid, per, true, true>(EngineDev, unsigned long long, uint32_t);   \
-    template __global__ void k_group<grid, per, false, true>(EngineDev, unsigned long long, uint32_t);
-NAER_GROUP(true, 1)
-NAER_GROUP(true, 4)
-NAER_GROUP(false, 1)
-NAER_GROUP(false, 4)
+// (deterministic aggregation in a cluster: one network, always one neuron a lane)
+#define NAER_GROUP(grid, per, det)                                                            \
+    template __global__ void k_group<grid, per, true, det>(EngineDev, unsigned long long, uint32_t); \
+    template __global__ void k_group<grid, per, false, det>(EngineDev, unsigned long long, uint32_t);
+NAER_GROUP(true, 1, false)
+NAER_GROUP(true, 4, false)
+NAER_GROUP(false, 1, false)
+NAER_GROUP(false, 4, false)
+NAER_GROUP(true, 1, true)
+NAER_GROUP(true, 4, true)
+NAER_GROUP(false, 1, true)
 #undef NAER_GROUP
 
 size_t group_smem_bytes(uint32_t own_neurons, uint32_t per_lane, bool rows, bool det) {
