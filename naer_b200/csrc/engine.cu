@@ -13,6 +13,7 @@
 
 #include "build_kernels.cuh"
 #include "engine.h"
+#include "group_plan.h"
 #include "philox.cuh"
 #include "sim_kernels.cuh"
 
@@ -1085,6 +1086,35 @@ static uint32_t group_own(const NetDev& d, const std::vector<PopDev>& pops, uint
     return (group_chunks(d, pops, per) + warps - 1) / warps * step_warps * 32 * per;
 }
 
+// What a network is expected to do in a grid step, from its description.  A
+// drive event that reaches the threshold by itself is a spike; inhibition
+// holds a driven population to about 0.6 of that, and to less the more inputs
+// a neuron has (plastic_indegree at 10 Hz: 7.7 Hz with 100 inputs, 4.4 with
+// 1,000, 3.6 with 4,000).  Within 0.84 to 1.32 of the events of the batches that
+// cluster_us was fitted to; recurrent excitation can saturate a network to 3 times the estimate.
+static Activity expected_activity(const NetDev& d, const NetHost& n, const std::vector<PopDev>& pops) {
+    bool inhibited = false;
+    for (const ConnSpec& c : n.conns)
+        inhibited = inhibited || c.csr || c.spec.weight < 0.0f || (c.spec.weight == 0.0f && c.spec.wmin < 0.0f);
+    const double dt = 1e-6 * d.dt_us;
+    double size = 0;
+    for (uint32_t x = 0; x < d.pop_count; ++x) size += pops[d.pop_first + x].size;
+    const double row = (double)n.synapses / size;
+    Activity a;
+    for (uint32_t x = 0; x < d.pop_count; ++x) {
+        const PopDev& p = pops[d.pop_first + x];
+        double rate = 8.0;
+        if (p.type == kPOISSON) rate = p.rate_hz;
+        else if (p.rate_hz > 0.0 && p.drive_w >= p.v_th && !inhibited) rate = p.rate_hz / (1.0 + p.rate_hz * p.t_ref_steps * dt);
+        else if (p.rate_hz > 0.0) rate = (1.0 + std::min(0.6 * p.rate_hz, 50.0)) / (inhibited ? 1.0 + row / 3000.0 : 1.0);
+        a.neurons += p.size;
+        a.drawn += p.rate_hz > 0.0 ? p.size : 0.0;
+        a.spikes += dt * rate * p.size;
+    }
+    a.events = a.spikes * row;
+    return a;
+}
+
 // Shared memory of a class; false if its blocks or clusters cannot be
 // resident.
 bool Engine::fit_class(GroupClass& c) {
@@ -1115,49 +1145,39 @@ bool Engine::fit_class(GroupClass& c) {
     return active >= 1;
 }
 
-// Geometry of k_group for one network, or false: k_step.  The lines below
-// were measured on B200,
-// µs per grid step, atomic aggregation; "k_step" includes its k_drive.
-//
-//   cluster of 16 blocks, 1 neuron a lane: at most one chunk a warp (two with
-//     windows of one step, up to 8M synapses).  LIF networks of 5k neurons /
-//     out-degree 100: 3.5 (grid 4.2, k_step 9.5); 12k / 100: 4.4 (4.6, 9.5);
-//     12k / 1000: 6.7 (6.0); plastic 12k / 300: 7.3 (8.4, 10.5); Brunel 5k:
-//     1.44 (1.55, 9.2), 10k: 2.2 (1.6, 9.4)
-//   grid, 1 neuron a lane up to two chunks a warp, else 4: 20k / 500: 5.1 (4 a
-//     lane 6.7, k_step 10.5); 100k / 1000: 9.2 (9.3, 12.0); 400k / 500: 13.9
-//     (12.4, 14.5); Brunel 40k: 3.4 (3.9, 10.4)
-//   k_step from 500k neurons (700k / 300: 17.0, grid 17.0; 1M / 1000: 27.0,
-//     27.4) or 250k with plasticity (300k / 300: 14.1, 14.1), unless windows
-//     are longer than one step
-//   deterministic aggregation (windows of one step, k_det_step where not):
-//     the same lines, except that the grid pays up to 250k neurons (200k /
-//     1000: 20.2, k_det_step 23.2; 400k / 500: 23.7, 25.2, but 400k / 1000:
-//     32.1, 27.0: k_det_step has a third more warps to wait for the events'
-//     exchanges), with plasticity up to 600k (300k / 300: 24.4, 29.9; 600k /
-//     200: 34.0, 36.2)
-//   block-local delivery (one barrier a step) up to 500k synapses a block: a
-//     block's share of a step's spikes varies, which costs more than the
-//     barrier saves once it is bound by its reductions (50k / 400: 6.6 against
-//     8.4 with the exchange; 200k / 1000: 11.8 against 11.0)
+static GroupNeed group_need(const NetDev& d, const NetHost& n, const std::vector<PopDev>& pops, bool det) {
+    GroupNeed g;
+    g.window = d.window;
+    g.stdp = d.stdp_on != 0;
+    g.det = det;
+    g.chunks = group_chunks(d, pops, 1);
+    g.synapses = n.synapses;
+    g.act = expected_activity(d, n, pops);
+    return g;
+}
+
+// Geometry of k_group for one network (single_form), or false: k_step or
+// k_det_step.
 bool Engine::plan_one(const std::vector<PopDev>& pops) {
     NetDev& d = h_nets_[0];
     const NetHost& n = *nets_[0];
     const bool det = aggregation_ == NAER_AGG_DETERMINISTIC;
-    const uint32_t step_warps = kGroupStepThreads / 32, chunks = group_chunks(d, pops, 1);
-    uint32_t c = 16;
-    const bool cluster = chunks <= c * step_warps ||
-                         (d.window == 1 && chunks <= 2 * c * step_warps && n.synapses <= 8000000ull);
-    if (!cluster) c = (uint32_t)sm_count_;
+    const uint32_t step_warps = kGroupStepThreads / 32;
+    const GroupNeed need = group_need(d, n, pops, det);
+    const GroupForm form = single_form(need, (uint32_t)sm_count_);
+    if (!form.group) return false;
+    const bool cluster = form.cluster;
+    const uint32_t c = cluster ? kGroupSingle : (uint32_t)sm_count_;
     if (c > kGroupMaxBlocks) return false;
     group_form_ = cluster ? kGroupCluster : kGroupGrid;
     GroupClass k;
     k.size = c;
     k.nets = 1;
-    k.per = cluster || chunks <= 2 * c * step_warps ? 1 : 4;
+    k.per = cluster || need.chunks <= 2 * c * step_warps ? 1 : 4;
     k.own = group_own(d, pops, c, k.per);
     k.stdp = d.stdp_on != 0;
     k.det = det;
+    d.local = form.local ? 1u : 0u;
     if (!cluster && (uint64_t)c * k.own * d.window > kGroupMostRecords)
         d.window = (uint32_t)std::max<uint64_t>(1, kGroupMostRecords / ((uint64_t)c * k.own));
     if (!cluster && d.window == 1 && n.n_storage > (det ? d.stdp_on ? 600000u : 250000u : d.stdp_on ? 250000u : 500000u))
@@ -1169,12 +1189,9 @@ bool Engine::plan_one(const std::vector<PopDev>& pops) {
 }
 
 // Clusters for several networks: every network gets the smallest cluster with
-// which its step takes at most T, for the T that minimises a launch's length.  The step times are a model
-// fitted to measurements (us, networks of 2k to 45k neurons on 1 to 16
-// blocks): the LIF's rounds of the warps, a chain of 1.3 (static) or 2.7
-// (plastic), and the events at the rates a block delivers them (800 and 260)
-// or the draws (880), whichever is longer.  False if the grid kernel, which
-// steps all networks together, is expected to be faster.
+// which its step takes at most T (cluster_us), for the T that minimises a
+// launch's length.  False if the grid kernel, which steps all networks together,
+// is expected to be faster (grid_us).
 bool Engine::plan_several(const std::vector<PopDev>& pops) {
     static const uint32_t sizes[] = {1, 2, 4, 8};  // clusters of 16 crowd the others out (20 of 5k: 8.3, without 7.0)
     constexpr int kSizes = 4;
@@ -1186,37 +1203,26 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
     NAER_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
     const size_t smem_most = (size_t)optin - 4096;  // less what the kernel declares itself
     std::vector<double> t(count * kSizes);
-    double plastic = 0, fixed = 0, neurons = 0;  // events per step, neurons
+    double events = 0, neurons = 0, ring_mb = 0;  // of all networks, a step
+    bool plastic = false;
     for (size_t i = 0; i < count; ++i) {
         const NetDev& d = h_nets_[i];
-        double spikes = 0, n = 0, drawn = 0;  // expected spikes per second
-        for (uint32_t x = 0; x < d.pop_count; ++x) {
-            const PopDev& p = pops[d.pop_first + x];
-            n += p.size;
-            drawn += p.rate_hz > 0.0 ? p.size : 0.0;
-            spikes += p.size * (p.type == kPOISSON ? p.rate_hz : p.rate_hz > 0.0 ? 1.0 + std::min(0.6 * p.rate_hz, 50.0) : 8.0);
-        }
-        const double ev = 1e-6 * d.dt_us * (double)nets_[i]->synapses * (spikes / n);
-        (d.stdp_on ? plastic : fixed) += ev;
-        neurons += n;
+        const GroupNeed need = group_need(d, *nets_[i], pops, false);
+        plastic = plastic || d.stdp_on;
+        events += need.act.events;
+        neurons += need.act.neurons;
+        ring_mb += 4e-6 * d.ring_slots * need.act.neurons;
         for (int k = 0; k < kSizes; ++k) {
             const uint32_t c = sizes[k], per = per_of(d, c);
             const double rounds = (double)group_own(d, pops, c, per) / (32.0 * per * step_warps);
-            const double lif = per == 1 ? 0.55 + 0.37 * rounds : 0.75 + 0.73 * rounds;
-            const double draw = drawn / c / 880.0;
-            const double rest = d.stdp_on ? 2.7 + std::max(1.8 + ev / (c * 260.0), draw)
-                                          : 1.3 + std::max(0.8 + ev / (c * 800.0), draw);
             // neurons that do not fit one block's shared memory
             const bool fits = group_smem_bytes(group_own(d, pops, c, per), per, false) <= smem_most;
-            t[i * kSizes + k] = fits ? lif + rest : 1e9;
+            t[i * kSizes + k] = fits ? cluster_us(need, c, per, rounds) : 1e9;
         }
     }
     // a launch as the device runs it: the clusters, largest first, each on
-    // free SMs for all its steps (clusters of mixed sizes leave some SMs of a
-    // GPC unused: with all 148 planned full, a cluster that finds no place
-    // waits for a whole launch: 40 networks of 30k 17.5 us, with 0.82 14.1)
-    const uint32_t sms = (uint32_t)(0.82 * sm_count_);
-    auto span_of = [&](const std::vector<int>& pick) {
+    // free SMs (of `sms`) for all its steps
+    auto span_of = [&](const std::vector<int>& pick, uint32_t sms) {
         std::vector<uint32_t> order(count);
         for (uint32_t i = 0; i < count; ++i) order[i] = i;
         std::sort(order.begin(), order.end(), [&](uint32_t l, uint32_t r) {
@@ -1227,6 +1233,7 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
         double now = 0, end = 0;
         for (uint32_t i : order) {
             const uint32_t c = sizes[pick[i]];
+            if (c > sms) return 1e30;
             while (free < c) {
                 now = busy.top().first;
                 free += busy.top().second;
@@ -1238,6 +1245,10 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
         }
         return end;
     };
+    // sizes are chosen for 0.82 of the SMs: clusters of mixed sizes leave some
+    // SMs of a GPC unused, and with all 148 planned full, a cluster that finds
+    // no place waits for a whole launch (40 networks of 30k 17.5 us, with 0.82
+    // 14.1)
     std::vector<double> targets(t);
     std::sort(targets.begin(), targets.end());
     double best = 1e30;
@@ -1249,18 +1260,20 @@ bool Engine::plan_several(const std::vector<PopDev>& pops) {
             while (k + 1 < kSizes && t[i * kSizes + k] > targets[x]) ++k;
             pick[i] = k;
         }
-        const double span = span_of(pick);
+        const double span = span_of(pick, (uint32_t)(0.82 * sm_count_));
         if (span < best && span < 1e8) {
             best = span;
             best_pick = pick;
         }
     }
-    const double grid = 8.0 + neurons / 3e5 + plastic / 8300.0 + fixed / 28000.0;
-    // measured, clusters / grid (model): 48 networks of up to 50k neurons 29.6 /
-    // 40.4 (21.7 / 39.5), 20 of 5k 7.0 / 10.8 (6.5 / 8.7), 100 of 20k 22.8 /
-    // 26.1 (18.0 / 25.2), 25 of 12k 11.8 / 12.2 (7.1 / 9.7), 10 of 30k 16.7 /
-    // 15.0 (14.0 / 13.3), 5 of 50k 20.5 / 13.0 (21.8 / 12.8)
-    if (best_pick.empty() || best > 0.95 * grid) return false;
+    if (best_pick.empty()) return false;
+    // the plan's length on the SMs that clusters of its sizes can use (15
+    // clusters of 8 run at a time: 32 networks in as many took three turns)
+    const bool even = std::count(best_pick.begin(), best_pick.end(), best_pick[0]) == (long)count;
+    const double usable = !even ? 0.85 : sizes[best_pick[0]] < 8 ? 1.0 : 0.82;
+    const double clusters = span_of(best_pick, (uint32_t)(usable * sm_count_));
+    const double grid = grid_us(neurons, events, ring_mb, plastic, tuning_.launch_steps);
+    if (!clusters_pay(clusters, grid)) return false;
     // classes by cluster size and neurons a lane, the largest clusters first
     group_classes_.clear();
     h_order_.clear();
@@ -1341,7 +1354,7 @@ void Engine::plan_group(const std::vector<PopDev>& pops) {
                 h_segs_.push_back(GroupSeg{d.g_first + f, std::min(seg, d.g_chunks - f), words + f * c.per, c.per, d.pop_first});
             d.seg_n = (uint32_t)h_segs_.size() - d.seg_first;
             words += d.g_chunks * c.per;
-            d.local = d.window == 1 && !d.stdp_on && !det && nets_[i]->synapses <= 500000ull * c.size ? 1u : 0u;
+            if (h_nets_.size() > 1) d.local = block_local(d.window, d.stdp_on != 0, nets_[i]->synapses, c.size) ? 1u : 0u;
             d.q_cap = group_own(d, pops, c.size, c.per) * d.window;
             d.q_off = group_entries_;
             group_entries_ += (uint64_t)d.q_cap * c.size;
