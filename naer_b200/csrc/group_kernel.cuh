@@ -32,12 +32,14 @@
 //
 // What bounds it: a step's chain of latencies (ring loads from L2, 350 to 770
 // cycles by die; a few hundred dependent instructions of one warp; row loads;
-// the reductions' fence; the barrier), not bytes: DRAM and the tensor-free
-// pipes are below 10 % busy.  Per grid step, against k_drive + k_step: 5k
-// neurons / out-degree 100: 3.5 against 9.5 us; 50k / in-degree 400: 5.4
-// against 11.0; 200k / 1000: 11.0 against 12.1; 100k plastic / 1000: 11.9
-// against 14.5; Brunel (delay 15 steps, called window by window) 2k: 1.7
-// against 8.6, 60k / 1.8e8 synapses: 7.1 against 17.0.
+// the reductions' fence; the barrier), not bytes: on the grid at 200k / 1000
+// DRAM is 2.5 % busy, L2 10 %, the SMs 17 %, and 14 of the 23 cycles between a
+// warp's instructions are waits at barriers.  Kernel time per grid step (events
+// around the launches), against k_drive + k_step: 5k neurons / out-degree 100:
+// 3.4 against 8.7 us; 50k / in-degree 400: 5.1 against 9.5; 200k / 1000: 11.0
+// against 12.0; 100k plastic / 1000: 11.0 against 13.0; Brunel (delay 15 steps,
+// called window by window) 2k: 1.8 against 8.5, 60k / 1.8e8 synapses: 6.3
+// against 12.6.
 namespace naer {
 
 constexpr uint32_t kGroupWarps = kGroupThreads / 32;
@@ -421,12 +423,11 @@ __device__ __forceinline__ void raster_end(const EngineDev& eng, unsigned long l
 // list of one event (most of them) nothing else.  A warp with more starts
 // than places goes over its rows a second time instead.
 // Bound by the same chain of latencies as the rest of k_group, with one
-// exchange and one head load more and the third barrier.  Per grid step,
-// against k_drive + k_det_step (whose fold reads the rows and links of all
-// events again, between barriers of two blocks an SM): 1k neurons /
-// out-degree 50: 6.0 against 10.5 us; 12k / 600: 12.5 against 17.9; 100k /
-// 500: 16.0 against 21.9; plastic 5k / 200: 8.4 against 21.4, 80k / 800: 14.7
-// against 27.7.
+// exchange and one head load more and the third barrier.  Kernel time per grid
+// step, against k_drive + k_det_step (whose fold reads the rows and links of all
+// events again, between barriers of two blocks an SM): 1k neurons / out-degree
+// 50: 6.1 against 10.3 us; 12k / 600: 12.5 against 18.1; 100k / 500: 16.7
+// against 22.1; plastic 5k / 200: 8.5 against 22.3, 80k / 800: 15.5 against 28.4.
 struct __align__(16) DetStart {
     uint32_t j, cell;
     float w;
@@ -564,8 +565,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     const bool drawer = wib >= kGroupSteppers;
     // the grid's drawing warps deliver too once they have drawn, with
     // plasticity: its items are one synapse a lane, each a chain of loads, and
-    // more warps keep more of them in flight (100k / 1000: 12.6 -> 11.9 us a
-    // step; static rows 14.5 and 14.6, so theirs stay with the others)
+    // more warps keep more of them in flight (100k / 1000, a pass of 1,000 steps
+    // with its results read: 12.6 -> 11.8 ms; of 500 steps with static rows, 200k
+    // / 1000: 7.23 and 7.32, so theirs stay with the others)
     constexpr bool kDrawersDeliver = kGrid && kPlastic && !kDet;
     const uint32_t nwarps = csz * kGroupSteppers, gw = rank * kGroupSteppers + wib;  // stepping warps
     Ctl* ctl = eng.ctl;
